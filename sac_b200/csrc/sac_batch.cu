@@ -54,6 +54,10 @@ struct sac_batch {
   void* P[4] = {nullptr, nullptr, nullptr, nullptr};
   double* BG = nullptr;
   double* dx = nullptr;
+  void* xr = nullptr;  // cell widths with their reciprocals (Stage2Args::xr)
+  long xr_off[3] = {0, 0, 0};
+  int axis_tab = 0;
+  bool widths_ok = true;
   double* drv = nullptr;  // driver profiles [2][totX] (users strat and tube)
   double* stg = nullptr;
   InstDyn* d_dyn = nullptr;
@@ -306,7 +310,10 @@ Stage2Args stage_base(sac_batch* b) {
   a.D = b->D;
   a.F = b->F;
   a.R = b->R;
-  a.dx = b->dx;
+  for (int d = 0; d < b->ndim; ++d) a.dx[d] = b->dx + (size_t)d * b->totX;
+  for (int d = 0; d < b->ndim; ++d) a.xr[d] = (const char*)b->xr + 2 * b->es * b->xr_off[d];
+  a.axis_tab = b->axis_tab;
+  a.general = b->widths_ok ? 0 : 1;
   a.gamma = b->par.gamma;
   for (int d = 0; d < 3; ++d) a.grav[d] = (d < b->ndim) ? b->par.grav[d] : 0.0;
   a.dmin = 0;
@@ -645,7 +652,7 @@ void free_all(sac_batch* b) {
     if (p) cudaFree((void*)p);
     p = nullptr;
   };
-  fr(b->BG), fr(b->dx), fr(b->drv), fr(b->stg), fr(b->d_dyn), fr(b->d_inst), fr(b->d_cour), fr(b->d_gh_all), fr(b->d_meshoff);
+  fr(b->BG), fr(b->dx), fr(b->xr), fr(b->drv), fr(b->stg), fr(b->d_dyn), fr(b->d_inst), fr(b->d_cour), fr(b->d_gh_all), fr(b->d_meshoff);
   fr(b->d_fused);
   fr(b->D), fr(b->F), fr(b->R), fr(b->d_type), fr(b->d_fixed), fr(b->d_fixB);
   for (Group& gr : b->groups) fr(gr.d_inst), fr(gr.d_face), fr(gr.d_nu), fr(gr.d_upd), fr(gr.d_gh);
@@ -708,7 +715,7 @@ sac_status sac_batch_create(const sac_params* p, int ndim, int ndir, int ninst, 
       sac_batch_destroy(b);
       return SAC_ERR_UNSUPPORTED;
     }
-    b->h_inst[i].o = Offs{off, off, 0, off};
+    b->h_inst[i].o = Offs{off, off, 0, off, {0, 0, 0}};
     off += g.ncell;
   }
   b->totP = b->totX = off;
@@ -758,6 +765,7 @@ sac_status sac_batch_set_grid(sac_batch* b, const double* x) {
   b->mindx2.assign((size_t)b->ninst * 3, 0.0);
   b->dtgrav.assign(b->ninst, kBig);
   long xoff = 0;
+  bool tab = true;
   for (int i = 0; i < b->ninst; ++i) {
     const Geom& g = b->h_inst[i].g;
     std::vector<double> hx1, hdx1;
@@ -770,6 +778,7 @@ sac_status sac_batch_set_grid(sac_batch* b, const double* x) {
         std::copy(prof.begin() + (long)k * g.ncell, prof.begin() + (long)(k + 1) * g.ncell,
                   hdrv.begin() + (long)k * b->totX + b->h_inst[i].o.X);
     }
+    tab = tab && widths_on_axes(g.n, g.lo, g.hi, ndim, g.ncell, hdx1.data());
     double mindx_all = kBig;
     for (int d = 0; d < ndim; ++d) {
       double m2 = kBig;
@@ -795,6 +804,28 @@ sac_status sac_batch_set_grid(sac_batch* b, const double* x) {
     BK(cudaMemset(p, 0, es * b->np * b->totP));  // scratch stages of finished instances stay finite
   }
   BK(cudaMalloc(&b->BG, sizeof(double) * (b->nw - b->np) * b->totP));
+  // the widths' table, per index along each dimension where every instance allows it
+  b->axis_tab = tab ? 1 : 0;
+  b->widths_ok = true;
+  std::vector<double> xr64;
+  std::vector<float> xr32;
+  for (int d = 0; d < ndim; ++d) {
+    const long first = (long)(b->prec == SAC_PREC_FP32 ? xr32.size() : xr64.size()) / 2;
+    b->xr_off[d] = first;
+    for (int i = 0; i < b->ninst; ++i) {
+      const Geom& g = b->h_inst[i].g;
+      const double* q = hdx.data() + (size_t)d * b->totX + b->h_inst[i].o.X;
+      b->h_inst[i].o.A[d] = (int)((long)(b->prec == SAC_PREC_FP32 ? xr32.size() : xr64.size()) / 2 - first);
+      if (b->prec == SAC_PREC_FP32)
+        append_width_pairs(xr32, g.n, g.lo, g.hi, ndim, g.ncell, q, d, tab);
+      else
+        b->widths_ok &= append_width_pairs(xr64, g.n, g.lo, g.hi, ndim, g.ncell, q, d, tab);
+    }
+  }
+  const size_t xr_bytes = xr64.size() * sizeof(double) + xr32.size() * sizeof(float);
+  BK(cudaMalloc(&b->xr, xr_bytes));
+  BK(cudaMemcpy(b->xr, xr64.empty() ? (const void*)xr32.data() : (const void*)xr64.data(), xr_bytes,
+                cudaMemcpyHostToDevice));
   BK(cudaMalloc(&b->dx, sizeof(double) * ndim * b->totX));
   BK(cudaMemcpy(b->dx, hdx.data(), sizeof(double) * hdx.size(), cudaMemcpyHostToDevice));
   if (gauss) {

@@ -32,6 +32,11 @@ using namespace sacgpu;
 
 namespace {
 constexpr double bigdouble = 1.0e99, smalldouble = 1.0e-99;
+// One cell in this many out of range (k_face) sends the FP64 3D update to the general
+// form's own kernels: at 128^3 its common kernel takes 0.67 ms per launch where no warp
+// meets such a cell and 2.2 where all do, those kernels 1.04 whatever the state, which is
+// even at 0.23 of the warps; the cells' stencils reach about twice as many
+constexpr long kQuietShare = 8;
 }
 
 struct sac_ctx {
@@ -52,10 +57,20 @@ struct sac_ctx {
   void* X = nullptr;  // cross-derivative half-sums (k_cross), allocated with hyperdiffusion
   double* x = nullptr;
   double* dx = nullptr;
+  void* xr = nullptr;  // cell widths with their reciprocals (Stage2Args::xr)
+  long xr_off[3] = {0, 0, 0};  // pairs before dimension d's
+  int axis_tab = 0;
+  bool widths_ok = true;  // the widths are in qdiv's range
   double* drv = nullptr;
   double* stg = nullptr;  // FP64 staging block for FP32 upload/download
   double drvA = 0.0;
-  unsigned long long* red = nullptr;  // 0..2 ctot, 3 maxnu, 4 courant, 5 divb max, 6 divb sq (as double)
+  // 0 maxnu, 1 courant, 2..4 ctot, 5 cells out of range of the last step (32 bits); then
+  // the FP64 stage's brick flags (one memset clears ctot and the flags)
+  unsigned long long* red = nullptr;
+  // that count on the host (pinned; FP64 3D) as of a recent step: it chooses between
+  // kernels with the same results, so its age does not matter
+  unsigned* h_nbad = nullptr;
+  size_t nflags = 0;  // bytes of flags (0: FP32)
   unsigned long long* kp = nullptr;   // keeppositive's words (smallfix only), see k_keeppos_scan
   int it_now = 0;                     // the step number last passed to sac_getdt or sac_advect
   double* fixB = nullptr;
@@ -188,13 +203,15 @@ bool grav_module(int u) {
 void release(sac_ctx* c) {
   for (auto& p : c->P)
     if (p) cudaFree(p), p = nullptr;
-  for (void* p : {(void*)c->BG, c->D, c->F, c->R, c->X, (void*)c->x, (void*)c->dx, (void*)c->drv,
+  for (void* p : {(void*)c->BG, c->D, c->F, c->R, c->X, (void*)c->x, (void*)c->dx, c->xr, (void*)c->drv,
                   (void*)c->stg, (void*)c->red, (void*)c->kp, (void*)c->fixB, (void*)c->d_type,
                   (void*)c->d_fixed})
     if (p) cudaFree(p);
   c->BG = c->x = c->dx = c->drv = c->stg = c->fixB = nullptr;
-  c->D = c->F = c->R = c->X = nullptr;
+  c->D = c->F = c->R = c->X = c->xr = nullptr;
   c->red = c->kp = nullptr;
+  if (c->h_nbad) cudaFreeHost(c->h_nbad);
+  c->h_nbad = nullptr;
   c->d_type = nullptr;
   c->d_fixed = nullptr;
 }
@@ -316,7 +333,7 @@ sac_status advect1_t(sac_ctx* c, const std::string& method, double qdt, int dmin
     const bool flux = (method == "cd4");
     const int u = c->par.user;
     const bool visc = c->par.sourceunsplit && visc_on(c);
-    CK(cudaMemsetAsync(c->red, 0, 3 * sizeof(unsigned long long), c->stream));
+    CK(cudaMemsetAsync(c->red + 2, 0, 4 * sizeof(unsigned long long) + c->nflags, c->stream));
     Stage2Args a{};
     a.g = g;
     a.wct = wct;
@@ -329,10 +346,16 @@ sac_status advect1_t(sac_ctx* c, const std::string& method, double qdt, int dmin
     a.F = c->F;
     a.R = c->R;
     a.X = c->X;
-    a.dx = c->dx;
+    const size_t pair = 2 * c->es;
+    for (int d = 0; d < g.ndim; ++d) a.xr[d] = (const char*)c->xr + pair * c->xr_off[d];
+    a.axis_tab = c->axis_tab;
+    a.flags = (unsigned char*)(c->red + 6);
+    a.fst[0] = 1;
+    a.fst[1] = (g.n[0] + 7) / 8;
+    a.fst[2] = a.fst[1] * ((g.n[1] + 7) / 8);
     a.drv = c->drv;
-    a.ctot = c->red;
-    a.maxnu = c->red + 3;
+    a.ctot = c->red + 2;
+    a.maxnu = c->red;
     a.qdt = qdt;
     // sources inside centdiff4 carry qdt*(idimmax-idimmin+1)/ndim, src/vaccd.t:73-75;
     // advect1 'source' passes qdt unchanged
@@ -343,6 +366,7 @@ sac_status advect1_t(sac_ctx* c, const std::string& method, double qdt, int dmin
     a.dmin = flux ? dmin : 1;
     a.dmax = flux ? dmax : 0;
     a.iwmask = mask;
+    a.general = a.dmin != 0 || a.dmax != g.ndim - 1 || mask != (1u << g.np) - 1u || !c->widths_ok;
     for (int d = 0; d < 3; ++d)
       for (int s2 = 0; s2 < 2; ++s2) a.zero1[d][s2] = c->zero1[d][s2];
     a.grav_on = (c->par.sourceunsplit && grav_module(u)) ? 1 : 0;
@@ -353,6 +377,12 @@ sac_status advect1_t(sac_ctx* c, const std::string& method, double qdt, int dmin
     a.res_compact = c->par.compactres ? 1 : 0;
     a.eta = c->par.eta;
     a.divb_on = (c->par.sourceunsplit && c->par.divbfix && g.ndim > 1) ? 1 : 0;
+    // the resistive terms divide products with eta and the step
+    if (a.res_on && (!(a.eta >= 0x1p-60 && a.eta <= 0x1p60) ||
+                     !(std::fabs(a.qdt2) >= 0x1p-80 && std::fabs(a.qdt2) <= 0x1p60)))
+      a.general = 1;
+    a.nbad = (unsigned*)(c->red + 5);
+    a.quiet = c->h_nbad && (long)*(volatile unsigned*)c->h_nbad > g.ncell / kQuietShare ? 1 : 0;
     a.driver = DRV_NONE;
     if (c->par.sourceunsplit && c->drv) {
       if (u == SAC_USR_SLOG && g.ndim == 3) {
@@ -882,14 +912,41 @@ sac_status sac_set_grid(sac_ctx* c, int ndim, int ndir, const int ixGhi[3], cons
   CK(cudaMalloc(&c->D, c->es * (ndir + 3) * N));
   CK(cudaMalloc(&c->F, c->es * (size_t)ndim * g.np * N));
   CK(cudaMalloc(&c->R, c->es * (size_t)nr_pairs(ndim) * N));
-  if (visc_on(c) && ndim > 1 && c->prec == SAC_PREC_FP64)  // the FP64 update reads them (k_cross)
+  if (visc_on(c) && ndim > 1)  // the update reads them (k_cross)
     CK(cudaMalloc(&c->X, c->es * (size_t)n_cross(ndim) * N));
   CK(cudaMalloc(&c->x, sizeof(double) * ndim * N));
   CK(cudaMalloc(&c->dx, sizeof(double) * ndim * N));
+  // the widths' table: per index along each dimension where they allow it
+  c->axis_tab = widths_on_axes(g.n, g.lo, g.hi, ndim, N, hdx.data()) ? 1 : 0;
+  c->widths_ok = true;
+  std::vector<double> xr64;
+  std::vector<float> xr32;
+  for (int d = 0; d < ndim; ++d) {
+    if (c->prec == SAC_PREC_FP32) {
+      c->xr_off[d] = (long)xr32.size() / 2;
+      append_width_pairs(xr32, g.n, g.lo, g.hi, ndim, N, hdx.data() + (size_t)d * N, d, c->axis_tab != 0);
+    } else {
+      c->xr_off[d] = (long)xr64.size() / 2;
+      c->widths_ok &= append_width_pairs(xr64, g.n, g.lo, g.hi, ndim, N, hdx.data() + (size_t)d * N, d, c->axis_tab != 0);
+    }
+  }
+  const size_t xr_bytes = xr64.size() * sizeof(double) + xr32.size() * sizeof(float);
+  CK(cudaMalloc(&c->xr, xr_bytes));
+  CK(cudaMemcpyAsync(c->xr, xr64.empty() ? (const void*)xr32.data() : (const void*)xr64.data(), xr_bytes,
+                     cudaMemcpyHostToDevice, c->stream));
   if (!hdrv.empty()) CK(cudaMalloc(&c->drv, sizeof(double) * 2 * N));
   if (c->prec == SAC_PREC_FP32) CK(cudaMalloc(&c->stg, sizeof(double) * g.np * N));
-  CK(cudaMalloc(&c->red, 8 * sizeof(unsigned long long)));
-  CK(cudaMemsetAsync(c->red, 0, 8 * sizeof(unsigned long long), c->stream));
+  c->nflags = 0;
+  if (c->prec == SAC_PREC_FP64) {
+    c->nflags = 1;
+    for (int d = 0; d < ndim; ++d) c->nflags *= (size_t)(g.n[d] + 7) / 8;
+  }
+  CK(cudaMalloc(&c->red, 6 * sizeof(unsigned long long) + c->nflags));
+  CK(cudaMemsetAsync(c->red, 0, 6 * sizeof(unsigned long long) + c->nflags, c->stream));
+  if (ndim == 3 && c->prec == SAC_PREC_FP64) {
+    CK(cudaMallocHost(&c->h_nbad, sizeof(unsigned)));
+    *c->h_nbad = 0;
+  }
   if (c->par.smallfix) {
     static const unsigned long long kp0[5] = {0, ~0ull, 0, 0, ~0ull};
     CK(cudaMalloc(&c->kp, sizeof(kp0)));
@@ -1192,7 +1249,7 @@ static sac_status getdt_impl(sac_ctx* c, double* dt, int it, bool static_scratch
         return fail(c, SAC_ERR_NONFINITE, "non-finite wave speed in getdt_courant");
       if (courantmax > smalldouble) d = std::min(d, c->par.courantpar / courantmax);
     } else if (c->par.courantpar > 0.0) {  // getdt_courant, src/vac.t:641-699
-      CK(cudaMemsetAsync(c->red + 4, 0, sizeof(unsigned long long), c->stream));
+      CK(cudaMemsetAsync(c->red + 1, 0, sizeof(unsigned long long), c->stream));
       const long nm = (long)(g.hi[0] - g.lo[0] + 1) * (g.hi[1] - g.lo[1] + 1) * (g.hi[2] - g.lo[2] + 1);
       const int bs = 256;
       const unsigned nb = (unsigned)std::min<long>((nm + bs - 1) / bs, 148L * 16);
@@ -1202,9 +1259,9 @@ static sac_status getdt_impl(sac_ctx* c, double* dt, int it, bool static_scratch
         using S = decltype(S0);
         const S* wp = (const S*)c->P[0];
         switch (g.ndir) {
-          case 1: k_courant<1, S><<<nb, bs, 0, c->stream>>>(g, wp, c->BG, c->dx, c->red + 4, c->par.gamma); break;
-          case 2: k_courant<2, S><<<nb, bs, 0, c->stream>>>(g, wp, c->BG, c->dx, c->red + 4, c->par.gamma); break;
-          default: k_courant<3, S><<<nb, bs, 0, c->stream>>>(g, wp, c->BG, c->dx, c->red + 4, c->par.gamma); break;
+          case 1: k_courant<1, S><<<nb, bs, 0, c->stream>>>(g, wp, c->BG, c->dx, c->red + 1, c->par.gamma); break;
+          case 2: k_courant<2, S><<<nb, bs, 0, c->stream>>>(g, wp, c->BG, c->dx, c->red + 1, c->par.gamma); break;
+          default: k_courant<3, S><<<nb, bs, 0, c->stream>>>(g, wp, c->BG, c->dx, c->red + 1, c->par.gamma); break;
         }
       };
       if (c->prec == SAC_PREC_FP32)
@@ -1213,7 +1270,7 @@ static sac_status getdt_impl(sac_ctx* c, double* dt, int it, bool static_scratch
         launch(0.0);
       }
       unsigned long long bits = 0;
-      CK(cudaMemcpyAsync(&bits, c->red + 4, sizeof(bits), cudaMemcpyDeviceToHost, c->stream));
+      CK(cudaMemcpyAsync(&bits, c->red + 1, sizeof(bits), cudaMemcpyDeviceToHost, c->stream));
       CK(cudaStreamSynchronize(c->stream));
       double courantmax;
       std::memcpy(&courantmax, &bits, sizeof(double));
@@ -1229,7 +1286,7 @@ static sac_status getdt_impl(sac_ctx* c, double* dt, int it, bool static_scratch
     if (grav_module(u)) {  // getdt_special of the Slog/gravity user files
       if (visc_on(c)) {    // getdt_visc, src/vacusr.viscosity.t:509-542
         unsigned long long bits = 0;
-        CK(cudaMemcpyAsync(&bits, c->red + 3, sizeof(bits), cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaMemcpyAsync(&bits, c->red, sizeof(bits), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
         double maxviscoef;
         std::memcpy(&maxviscoef, &bits, sizeof(double));
@@ -1239,7 +1296,7 @@ static sac_status getdt_impl(sac_ctx* c, double* dt, int it, bool static_scratch
           const double m = (maxviscoef + 0.0) / c->mindx2[dd];  // = max over the mesh of (maxviscoef/dx^2)
           d = std::min(d, c->par.dtdiffpar / m);
         }
-        CK(cudaMemsetAsync(c->red + 3, 0, sizeof(unsigned long long), c->stream));
+        CK(cudaMemsetAsync(c->red, 0, sizeof(unsigned long long), c->stream));
       }
       // getdt_grav, src/vacusr.gravity.t:97-138 (evaluated at it==itmin only)
       if (it == c->itmin) {
@@ -1374,6 +1431,8 @@ sac_status sac_advect(sac_ctx* c, const char* method, const int* iws, int idimmi
     return fail(c, SAC_ERR_UNSUPPORTED, "typeadvance=" + ta);
   }
 #undef RUN
+  if (c->h_nbad)
+    CK(cudaMemcpyAsync(c->h_nbad, c->red + 5, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaGetLastError());
   return SAC_OK;
 }
@@ -1427,10 +1486,10 @@ sac_status sac_diag(sac_ctx* c, sac_diag_out* out) {
   });
   out->divb_l2 = std::sqrt(s2 / (double)n);
   out->divb_linf = mx;
-  unsigned long long bits[8];
+  unsigned long long bits[5];
   CK(cudaMemcpy(bits, c->red, sizeof(bits), cudaMemcpyDeviceToHost));
-  std::memcpy(&out->maxviscoef, &bits[3], sizeof(double));
-  for (int d = 0; d < 3; ++d) std::memcpy(&out->ctot[d], &bits[d], sizeof(double));
+  std::memcpy(&out->maxviscoef, &bits[0], sizeof(double));
+  for (int d = 0; d < 3; ++d) std::memcpy(&out->ctot[d], &bits[2 + d], sizeof(double));
   out->nonfinite = nonfinite;
   if (c->kp) {
     unsigned long long kp[5];

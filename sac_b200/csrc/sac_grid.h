@@ -5,6 +5,7 @@
 #pragma once
 #include <cmath>
 #include <cstdlib>
+#include <cstring>
 #include <vector>
 
 namespace sacgpu {
@@ -78,6 +79,75 @@ inline void gridsetup1(const int n[3], const int lo[3], const int hi[3], int ndi
           m[d] -= 1;
           hdx[d * ncell + gid(i, j, k)] = 0.5 * (qx[d * qc + qid(p[0], p[1], p[2])] - qx[d * qc + qid(m[0], m[1], m[2])]);
         }
+}
+
+// The rows of dimension d's table of widths: row 0 over the mesh, then one for each
+// ghost layer next to the mesh across d (getcurrent reads the widths there, and
+// gridsetup1's extrapolation rounds the coordinates along d in them), lower and upper
+// of every other dimension in order.  Row r holds the cells with the coordinates
+// a..b in the dimensions other than d.
+inline void width_row(const int lo[3], const int hi[3], int d, int r, int a[3], int b[3]) {
+  for (int e = 0; e < 3; ++e) a[e] = lo[e], b[e] = hi[e];
+  if (r > 0) {
+    const int k = (r - 1) / 2, e = k < d ? k : k + 1;
+    a[e] = b[e] = (r - 1) % 2 ? hi[e] + 1 : lo[e] - 1;
+  }
+}
+
+// Whether the width of every dimension varies along that dimension alone (bit for
+// bit) in each of those rows, so that one entry per index and row holds it.
+inline bool widths_on_axes(const int n[3], const int lo[3], const int hi[3], int ndim, long ncell,
+                           const double* hdx) {
+  const long st[3] = {1, n[0], (long)n[0] * n[1]};
+  for (int d = 0; d < ndim; ++d)
+    for (int r = 0; r < 2 * ndim - 1; ++r) {
+      const double* q = hdx + (size_t)d * ncell;
+      int a[3], b[3];
+      width_row(lo, hi, d, r, a, b);
+      const long first = a[0] + st[1] * a[1] + st[2] * a[2] - st[d] * a[d];  // index 0 along d
+      a[d] = 0;
+      b[d] = n[d] - 1;
+      for (int k = a[2]; k <= b[2]; ++k)
+        for (int j = a[1]; j <= b[1]; ++j) {
+          const double* row = q + st[1] * j + st[2] * k;
+          bool same = true;
+          if (d == 0) {
+            same = std::memcmp(row, q + first, sizeof(double) * n[0]) == 0;
+          } else {
+            const double v = q[first + st[d] * (d == 1 ? j : k)];
+            for (int i = a[0]; i <= b[0]; ++i) same &= row[i] == v;
+          }
+          if (!same) return false;
+        }
+    }
+  return true;
+}
+
+// (dx, 1/dx) pairs of S, appended to out: the rows above (tab), or one per cell.
+// False where a width is outside the range of the stage's divisions through its
+// reciprocal (qdiv, out_of_range).
+template <typename S>
+inline bool append_width_pairs(std::vector<S>& out, const int n[3], const int lo[3], const int hi[3], int ndim,
+                               long ncell, const double* q, int d, bool tab) {
+  const long st[3] = {1, n[0], (long)n[0] * n[1]};
+  bool in_range = true;
+  auto put = [&](double v) {
+    in_range = in_range && v >= 0x1p-40 && v <= 0x1p40;
+    out.push_back((S)v);
+    out.push_back((S)(1.0 / v));
+  };
+  if (!tab) {
+    out.reserve(out.size() + 2 * ncell);
+    for (long i = 0; i < ncell; ++i) put(q[i]);
+    return in_range;
+  }
+  for (int r = 0; r < 2 * ndim - 1; ++r) {
+    int a[3], b[3];
+    width_row(lo, hi, d, r, a, b);
+    const long first = a[0] + st[1] * a[1] + st[2] * a[2] - st[d] * a[d];
+    for (long i = 0; i < n[d]; ++i) put(q[first + st[d] * i]);
+  }
+  return in_range;
 }
 
 // Spatial profiles of the Gaussian velocity drivers on the full grid, two

@@ -36,9 +36,11 @@ struct Geom {
 
 // Offsets of one grid's blocks inside the arrays of the four families: advanced
 // state (P: w, w1, w2, w3), background (B), per-stage intermediates (I: D, F, R)
-// and grid (X: dx, driver profiles).  A single grid has all offsets 0.
+// and grid (X: dx, driver profiles; A: the axis tables of the cell widths, one
+// entry per index along a dimension).  A single grid has all offsets 0.
 struct Offs {
   long P, B, I, X;
+  int A[3];
 };
 
 // ---- many independent grids (the batched path) -----------------------------
@@ -105,6 +107,56 @@ __device__ __forceinline__ double dvs_rn(double n, double d) {
   return __ddiv_rn(n, d);
 }
 __device__ __forceinline__ float dvs_rn(float n, float d) { return __fdiv_rn(n, d); }
+
+// ---- divisions by a divisor whose reciprocal is at hand -------------------
+// Correctly rounded n / d from r = RN(1/d): q = RN(n r), e = n - q d, RN(q + e r)
+// (Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990): one multiply and two FMAs instead of the divide's reciprocal
+// iteration, and no slow path, whose branch keeps the loads behind it from being
+// issued ahead.  e has to be exact and q normal: n zero (the quotient is then a zero,
+// whose sign may differ from the divide's) or at least 2^-969 in magnitude.
+__device__ __forceinline__ double div_markstein(double n, double d, double r) {
+  const double q = __dmul_rn(n, r);
+  const double e = __fma_rn(-q, d, n);
+  return __fma_rn(e, r, q);
+}
+
+// n / d with r = RN(1/d).  FAST: Markstein's form, for cells whose fields are in range
+// (out_of_range below); otherwise the divide.  FP32 storage multiplies by the
+// reciprocal in both (1.5 ulp at most; the approximate divide has 2), except in a unit
+// that keeps IEEE rules for it (SAC_F32_IEEE_DIV).
+template <bool FAST>
+__device__ __forceinline__ double qdiv(double n, double d, double r) {
+  if constexpr (FAST) return div_markstein(n, d, r);
+  else return n / d;
+}
+template <bool FAST>
+__device__ __forceinline__ float qdiv(float n, float d, float r) {
+#ifdef SAC_F32_IEEE_DIV
+  return n / d;
+#else
+  return n * r;
+#endif
+}
+
+// A field value outside {0} and [2^-200, 2^100) in magnitude, NaN and Inf included.
+// With a cell's and its stencil's fields inside, the total density nonzero and c_tot
+// and the widths in their ranges, every numerator of the stage is zero or at least
+// 2^-859: the smallest are gradient4's of the energy flux (products of three fields,
+// 2^-600, over a density of 2^100, with 53 bits of cancellation in the product sum, in
+// the flux and in the difference) and the differences of a momentum times a viscous
+// flux (2^-200 * 2^-593: a velocity difference 2^-353 over a width of 2^40, c_tot
+// 2^-100, setnu's quotient 2^-60 and a width 2^-40).
+constexpr unsigned kRangeLo = (1023u - 200u) << 20, kRangeHi = (1023u + 100u) << 20;
+__device__ __forceinline__ bool out_of_range(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu;
+  return (hi - kRangeLo) >= (kRangeHi - kRangeLo) && x != 0.0;
+}
+
+// setnu's c_tot (the bits of a maximum of wave speeds) outside {0} and [2^-100, 2^200]
+__device__ __forceinline__ bool ctot_out_of_range(unsigned long long bits) {
+  return bits != 0ull && (bits < ((1023ull - 100) << 52) || bits > ((1023ull + 200) << 52));
+}
 
 __device__ __forceinline__ void atomic_max_nonneg(unsigned long long* a, double v) {
   // non-negative doubles order like their bit patterns; NaN maps above +Inf

@@ -48,30 +48,63 @@ __device__ __forceinline__ S ldt(const S* p, I i) {
 // ---------------------------------------------------------------------------
 // per-cell bodies (one grid, located by the offsets o)
 // ---------------------------------------------------------------------------
+// (width, reciprocal) of dimension d: from the axis table at index pd along d, or
+// per cell at cc
+template <typename S>
+__device__ __forceinline__ void width_at(const Stage2Args& a, const Offs& o, int d, int pd, long cc, S& dx, S& rx) {
+  const long i = a.axis_tab ? (long)(o.A[d] + pd) : o.X + cc;
+  if constexpr (sizeof(S) == 8) {
+    const double2 v = __ldg((const double2*)a.xr[d] + i);
+    dx = v.x, rx = v.y;
+  } else {
+    const float2 v = __ldg((const float2*)a.xr[d] + i);
+    dx = v.x, rx = v.y;
+  }
+}
+
 // the k_face arithmetic of the cell whose fields are read at c: dout(i, v) takes
 // the derived field i, fout(d, iw, v) the flux of iw along d for the dimensions in
-// the bit mask fdims; mesh tells whether the getcmax maxima apply there
+// the bit mask fdims; mesh tells whether the getcmax maxima apply there.
+//
+// Every quotient has the total density as its divisor: one reciprocal and the
+// three-operation form (qdiv) instead of about 30 divides per cell.  A cell with a
+// field out of range takes the divide, and is reported (FP64 storage; FP32 values
+// squared or cubed stay inside the range of FP64).  Measured with the update's form
+// of the same (launch_update).
 template <int NDIM, int NDIR, typename S, class DOut, class FOut>
-__device__ __forceinline__ void face_eval(const Stage2Args& a, const Offs& o, long c, bool mesh, double gamma,
-                                          double* cm, unsigned fdims, DOut&& dout, FOut&& fout) {
+__device__ __forceinline__ bool face_eval(const Stage2Args& a, const Offs& o, long c, bool mesh, double gamma,
+                                          double* cm, unsigned fdims, bool test, DOut&& dout, FOut&& fout) {
   constexpr int E = NDIR + 1;
   auto W = [&](int iw) { return (const S*)a.fW[iw] + o.P; };
   auto BG = [&](int i) { return a.fBG[i] + o.B; };
-  {
-    const double rho = (double)W(0)[c];
-    const double eb = BG(0)[c];
-    const double rhob = BG(1)[c];
-    const double rt = rho + rhob;
-    double m[NDIR], b[NDIR], bg[NDIR], v[NDIR];
+  const double rho = (double)W(0)[c];
+  const double eb = BG(0)[c];
+  const double rhob = BG(1)[c];
+  const double rt = rho + rhob;
+  double m[NDIR], b[NDIR], bg[NDIR];
 #pragma unroll
-    for (int C = 0; C < NDIR; ++C) {
-      m[C] = (double)W(1 + C)[c];
-      b[C] = (double)W(E + 1 + C)[c];
-      bg[C] = BG(2 + C)[c];
-    }
-    const double e = (double)W(E)[c];
+  for (int C = 0; C < NDIR; ++C) {
+    m[C] = (double)W(1 + C)[c];
+    b[C] = (double)W(E + 1 + C)[c];
+    bg[C] = BG(2 + C)[c];
+  }
+  const double e = (double)W(E)[c];
+  bool bad = false;
+  if (sizeof(S) == 8 && test) {
+    bad = !(fabs(rt) >= 0x1p-100 && fabs(rt) < 0x1p100) || out_of_range(rho) || out_of_range(e) || out_of_range(eb) || out_of_range(rhob);
 #pragma unroll
-    for (int C = 0; C < NDIR; ++C) v[C] = dvs_rn(m[C], rt);  // getv / tmp_nu for m
+    for (int C = 0; C < NDIR; ++C) bad = bad || out_of_range(m[C]) || out_of_range(b[C]) || out_of_range(bg[C]);
+  }
+  auto body = [&](auto fastc) {
+    constexpr bool FAST = decltype(fastc)::value;
+    const double rr = FAST ? __drcp_rn(rt) : 0.0;
+    auto by_rt = [&](double n) {
+      if constexpr (FAST) return div_markstein(n, rt, rr);
+      else return dvs_rn(n, rt);
+    };
+    double v[NDIR];
+#pragma unroll
+    for (int C = 0; C < NDIR; ++C) v[C] = by_rt(m[C]);  // getv / tmp_nu for m
     double b2 = 0.0, m2 = 0.0, bb = 0.0;
 #pragma unroll
     for (int C = 0; C < NDIR; ++C) {
@@ -83,10 +116,10 @@ __device__ __forceinline__ void face_eval(const Stage2Args& a, const Offs& o, lo
 #pragma unroll
     for (int C = 0; C < NDIR; ++C) dout(1 + C, (S)v[C]);
     // tmp_nu for iw=173, src/vacusr.viscosity.t:301
-    dout(NDIR + 1, (S)sub_rn(e, mul_rn(0.5, add_rn(b2, dvs_rn(m2, rt)))));
+    dout(NDIR + 1, (S)sub_rn(e, mul_rn(0.5, add_rn(b2, by_rt(m2)))));
     // getptotal, src/vacphys0.t.mhd:199-201
     const double pp = (gamma - 2.0) * (bb + 0.5 * b2);
-    const double ptot = (gamma - 1.0) * (e - dvs(0.5 * m2, rt)) - pp;
+    const double ptot = (gamma - 1.0) * (e - by_rt(0.5 * m2)) - pp;
     dout(NDIR + 2, (S)ptot);
     // fluxes in the storage precision's arithmetic (FP64 for the FP64 path; FP32
     // for the FP32 path, whose pressure/energy recovery above stays FP64)
@@ -99,7 +132,11 @@ __device__ __forceinline__ void face_eval(const Stage2Args& a, const Offs& o, lo
       bgC[C] = (C_)bg[C];
       vC[C] = (C_)v[C];
     }
-    const C_ rtC = (C_)rt, ptC = (C_)ptot, ebC = (C_)eb, eC = (C_)e, rhoC = (C_)rho, rhobC = (C_)rhob;
+    [[maybe_unused]] const C_ rtC = (C_)rt, rrC = (C_)rr, ptC = (C_)ptot, ebC = (C_)eb, eC = (C_)e, rhoC = (C_)rho, rhobC = (C_)rhob;
+    auto by_rtC = [&](C_ n) {
+      if constexpr (sizeof(S) == 8) return by_rt(n);
+      else return qdiv<true>(n, rtC, rrC);
+    };
     C_ s1 = C_(0), s2 = C_(0);
 #pragma unroll
     for (int C = 0; C < NDIR; ++C) s1 = s1 + bgC[C] * mC[C];
@@ -109,7 +146,7 @@ __device__ __forceinline__ void face_eval(const Stage2Args& a, const Offs& o, lo
     for (int d = 0; d < NDIM; ++d) {
       if (!((fdims >> d) & 1u)) continue;
       const C_ vd = vC[d], bd = bC[d], bgd = bgC[d], md = mC[d];
-      fout(d, 0, (S)(dvs(rhobC * md, rtC) + vd * rhoC));
+      fout(d, 0, (S)(by_rtC(rhobC * md) + vd * rhoC));
 #pragma unroll
       for (int C = 0; C < NDIR; ++C) {
         C_ f;
@@ -119,7 +156,7 @@ __device__ __forceinline__ void face_eval(const Stage2Args& a, const Offs& o, lo
           f = -(bC[C] * bgd + bd * bgC[C]) - bC[C] * bd;
         fout(d, 1 + C, (S)(f + vd * mC[C]));
       }
-      const C_ fe = dvs(md * (ptC + C_(0)) - bd * s1 - bgd * s2, rtC) + dvs(ebC * md, rtC) - dvs(bd * s2, rtC);
+      const C_ fe = by_rtC(md * (ptC + C_(0)) - bd * s1 - bgd * s2) + by_rtC(ebC * md) - by_rtC(bd * s2);
       fout(d, E, (S)(fe + vd * eC));
       // b_d has no flux along d (getflux sets transport=.false., src/vacphys.mhd0.t:204-206), and
       // k_update never reads that slot, so it is not written
@@ -128,64 +165,86 @@ __device__ __forceinline__ void face_eval(const Stage2Args& a, const Offs& o, lo
         if (C != d) fout(d, E + 1 + C, (S)(-(vC[C] * (bd + bgd)) + vd * bgC[C] + vd * bC[C]));
     }
     if (mesh) {
-        // getpthermal, getcsound2, getcmax: src/vacphys0.t.mhd:95-183
-        double q = 0.5 * m2 / rt;
-        q = q + 0.5 * b2 + bb;
-        const double p = (gamma - 1.0) * (e - q);
-        double bgs = 0.0, Bt2 = 0.0;
+      // getpthermal, getcsound2, getcmax: src/vacphys0.t.mhd:95-183
+      double q = by_rt(0.5 * m2);
+      q = q + 0.5 * b2 + bb;
+      const double p = (gamma - 1.0) * (e - q);
+      double bgs = 0.0, Bt2 = 0.0;
 #pragma unroll
-        for (int C = 0; C < NDIR; ++C) bgs = bgs + bg[C] * bg[C];
-        const double cs2 = gamma * (p + (gamma - 1.0) * (eb - 0.5 * bgs)) / rt;
+      for (int C = 0; C < NDIR; ++C) bgs = bgs + bg[C] * bg[C];
+      const double cs2 = by_rt(gamma * (p + (gamma - 1.0) * (eb - 0.5 * bgs)));
 #pragma unroll
-        for (int C = 0; C < NDIR; ++C) {
-          const double B = b[C] + bg[C];
-          Bt2 = Bt2 + B * B;
-        }
-        const double cf2 = Bt2 / rt + cs2;
+      for (int C = 0; C < NDIR; ++C) {
+        const double B = b[C] + bg[C];
+        Bt2 = Bt2 + B * B;
+      }
+      const double cf2 = by_rt(Bt2) + cs2;
 #pragma unroll
-        for (int d = 0; d < NDIM; ++d) {
-          const double Bd = b[d] + bg[d];
-          cm[d] = sqrt(0.5 * (cf2 + sqrt(cf2 * cf2 - 4.0 * cs2 * (Bd * Bd) / rt))) + fabs(m[d] / rt);
-        }
+      for (int d = 0; d < NDIM; ++d) {
+        const double Bd = b[d] + bg[d];
+        cm[d] = sqrt(0.5 * (cf2 + sqrt(cf2 * cf2 - by_rt(4.0 * cs2 * (Bd * Bd))))) + fabs(v[d]);
+      }
     }
-  }
+  };
+  if (sizeof(S) == 8 && (bad || a.quiet))
+    body(std::false_type{});
+  else
+    body(std::true_type{});
+  return bad;
 }
 
 // k_face body at local cell c: the derived fields and every flux into D and F
 template <int NDIM, int NDIR, typename S>
-__device__ __forceinline__ void face_cell(const Stage2Args& a, const Offs& o, int c, bool mesh, double gamma,
-                                          double* cm) {
-  face_eval<NDIM, NDIR, S>(
-      a, o, c, mesh, gamma, cm, (1u << NDIM) - 1u, [&](int i, S v) { ((S*)a.fD[i] + o.I)[c] = v; },
+__device__ __forceinline__ bool face_cell(const Stage2Args& a, const Offs& o, int c, bool mesh, double gamma,
+                                          double* cm, bool test = true) {
+  return face_eval<NDIM, NDIR, S>(
+      a, o, c, mesh, gamma, cm, (1u << NDIM) - 1u, test, [&](int i, S v) { ((S*)a.fD[i] + o.I)[c] = v; },
       [&](int d, int iw, S v) { ((S*)a.fF[d][iw] + o.I)[c] = v; });
 }
 
-// setnu's face quotient from a window of six values of q along one dimension
-// (TILE: q is a shared-memory tile)
-template <bool TILE = false, typename S>
-__device__ __forceinline__ S face_quotient(const S* __restrict__ q, int c, int s, int pos, int lo, int hi, S pre) {
-  // q(c-2..c+3) along s; the layer beyond the two ghosts is the mirror image
-  // about the first/last mesh cell (tmp_nuI, src/vacusr.viscosity.t:378-400)
-  S a[6];
+// max(m, x) for m >= 0 that ignores a NaN x, as fmax does: in FP64 a compare and a
+// select, half the instructions of fmax
+__device__ __forceinline__ double max_from(double m, double x) { return x > m ? x : m; }
+__device__ __forceinline__ float max_from(float m, float x) { return fmaxf(m, x); }
+
+// cell indices of setnu's window q(c-2..c+3) along one dimension (stride s, local
+// coordinate pos): the layer beyond the two ghosts is the mirror image about the
+// first/last mesh cell (tmp_nuI, src/vacusr.viscosity.t:378-400)
+__device__ __forceinline__ void face_offsets(int c, int s, int pos, int lo, int hi, int off[6]) {
 #pragma unroll
   for (int o = -2; o <= 3; ++o) {
     int p = pos + o;
     if (p <= lo - 3) p = lo + 3;
     if (p >= hi + 3) p = hi - 3;
-    a[o + 2] = ldt<TILE>(q, c + (p - pos) * s);
+    off[o + 2] = c + (p - pos) * s;
   }
-  S d1[5], d3[3];
+}
+
+template <typename S>
+__device__ __forceinline__ S face_d3(S a0, S a1, S a2, S a3) {  // d3R, src/vacusr.viscosity.t:413
+  return fabsT(sub_rn(mul_rn(S(3), sub_rn(a2, a1)), sub_rn(a3, a0)));
+}
+
+// max|d3R| and max|d1R| of a window of q (TILE: q is a shared-memory tile); md1 is 0
+// and md3 NaN where every difference is NaN
+template <bool TILE, typename S>
+__device__ __forceinline__ void face_maxima(const S* __restrict__ q, const int off[6], S& md3, S& md1) {
+  S a[6];
 #pragma unroll
-  for (int j = 0; j < 5; ++j) d1[j] = fabsT(a[j + 1] - a[j]);  // d1R(c-2+j), :414
+  for (int o = 0; o < 6; ++o) a[o] = ldt<TILE>(q, off[o]);
+  md1 = S(0);
 #pragma unroll
-  for (int j = 0; j < 3; ++j)  // d3R(c-1+j), :413
-    d3[j] = fabsT(sub_rn(mul_rn(S(3), sub_rn(a[j + 2], a[j + 1])), sub_rn(a[j + 3], a[j])));
-  const S md3 = fmaxT(fmaxT(d3[0], d3[1]), d3[2]);
-  const S md1 = fmaxT(fmaxT(fmaxT(fmaxT(d1[0], d1[1]), d1[2]), d1[3]), d1[4]);
-  // zero where the window is flat (md1 == 0): branch before dividing, since 0/0
-  // leaves the division's fast path, and a state at rest is flat almost everywhere
+  for (int j = 0; j < 5; ++j) md1 = max_from(md1, fabsT(a[j + 1] - a[j]));  // d1R(c-2+j), :414
+  md3 = fmaxT(fmaxT(face_d3(a[0], a[1], a[2], a[3]), face_d3(a[1], a[2], a[3], a[4])), face_d3(a[2], a[3], a[4], a[5]));
+}
+
+// setnu's face quotient c_tot*c_hyp*md3R/md1R (:424) from the window's maxima; zero
+// where the window is flat (md1 == 0): branch before dividing, since 0/0 leaves the
+// division's fast path, and a state at rest is flat almost everywhere
+template <typename S>
+__device__ __forceinline__ S face_ratio(S pre, S md3, S md1) {
   if (!(md1 > S(0))) return S(0);
-  return pre * md3 / md1;  // c_tot*c_hyp*md3R/md1R, :424
+  return pre * md3 / md1;
 }
 
 // k_nu body at local cell c with local coordinates p: every setnu pair's face
@@ -197,20 +256,24 @@ __device__ __forceinline__ void nu_cell(const Stage2Args& a, const Geom& g, cons
   constexpr int E = NDIR + 1;
 #pragma unroll
   for (int k = 0; k < NDIM; ++k) {
-    const int s = (int)g.st[k];
-    const int pos = p[k], lo = g.lo[k], hi = g.hi[k];
+    int off[6];
+    face_offsets(c, (int)g.st[k], p[k], g.lo[k], g.hi[k], off);
     const double ct = __longlong_as_double((long long)ctot[k]);
     // c_hyp: 0.04 for rho, the "173" energy and b; 0.4 for the momenta (:284-290)
     const S p04 = (S)(ct * 0.04), p4 = (S)(ct * 0.4);
-    auto Qw = [&](int ip) { return (S*)a.fQ[ip] + o.I; };
     auto W = [&](int iw) { return (const S*)a.fW[iw] + o.P; };
     auto Df = [&](int i) { return (const S*)a.fD[i] + o.I; };
-    Qw(PR::rho(k))[c] = face_quotient(W(0), c, s, pos, lo, hi, p04);
-    Qw(PR::e(k))[c] = face_quotient(Df(NDIR + 1), c, s, pos, lo, hi, p04);
+    auto quotient = [&](int pair, const S* q, S pre) {
+      S md3, md1;
+      face_maxima<false>(q, off, md3, md1);
+      ((S*)a.fQ[pair] + o.I)[c] = face_ratio(pre, md3, md1);
+    };
+    quotient(PR::rho(k), W(0), p04);
+    quotient(PR::e(k), Df(NDIR + 1), p04);
 #pragma unroll
     for (int l = 0; l < NDIM; ++l) {
-      Qw(PR::v(l, k))[c] = face_quotient(Df(1 + l), c, s, pos, lo, hi, p4);
-      if (l != k) Qw(PR::b(l, k))[c] = face_quotient(W(E + 1 + l), c, s, pos, lo, hi, p04);
+      quotient(PR::v(l, k), Df(1 + l), p4);
+      if (l != k) quotient(PR::b(l, k), W(E + 1 + l), p04);
     }
   }
 }
@@ -234,10 +297,11 @@ struct TileView {
 // single-grid path); without it the update computes them at both neighbours.
 // OPT_RES1: the resistive source in the compact form addsource_res1 instead of
 // addsource_res2's (OPT_RES); the two are never combined.
-// OPT_PART_A / OPT_PART_B: the update in two launches, cut after centdiff4 and
-// gravity; part A stores the partial sums in the stage's output array, part B
-// continues from them at the same cell, so every addition keeps its order.
-enum StageOpt { OPT_DIVB = 1, OPT_RES = 2, OPT_PRE = 4, OPT_RES1 = 8, OPT_PART_A = 16, OPT_PART_B = 32 };
+// OPT_QUIET: the general form for every cell, at the occupancy that suits it.
+// OPT_PART_A / OPT_PART_B (with OPT_QUIET): the update in two launches, cut after
+// centdiff4 and gravity; part A stores the partial sums in the stage's output array,
+// part B continues from them at the same cell, so every addition keeps its order.
+enum StageOpt { OPT_DIVB = 1, OPT_RES = 2, OPT_PRE = 4, OPT_RES1 = 8, OPT_QUIET = 16, OPT_PART_A = 32, OPT_PART_B = 64 };
 
 // Levi-Civita symbol of 0-based indices (lvc, src/vacdef.t:91)
 __host__ __device__ constexpr int lvc3(int i, int j, int k) {
@@ -254,12 +318,19 @@ __host__ __device__ constexpr int res_idirmin(int ndim, int ndir) {
   return m;
 }
 
-// k_update body at the mesh cell pos
-template <int NDIM, int NDIR, typename S, int OPT, bool TILE = false>
+// k_update body at the mesh cell pos.  FAST: an unsplit sweep over every advanced
+// variable, the divisions by the cell widths and by 12 in their three-operation form
+// (qdiv), for cells whose stencil's fields are in range.
+//
+// The terms are written without branches around their loads (zero rules select
+// after the arithmetic): the FP64 update is bound by the latency of its ~200 loads
+// per cell, and a branch around a load, or a divide's slow path, keeps the loads
+// behind it from being issued before it.
+template <int NDIM, int NDIR, typename S, int OPT, bool FAST, bool TILE = false>
 __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, const Offs& o, const int pos[3],
                                             double qdt_d, double qdt2_d, double tdep, double drvA,
                                             double& numax_out, const TileView<S>* tv = nullptr) {
-  static_assert(!TILE || (OPT & (OPT_DIVB | OPT_RES | OPT_RES1 | OPT_PRE | OPT_PART_A | OPT_PART_B)) == 0,
+  static_assert(!TILE || (OPT & (OPT_DIVB | OPT_RES | OPT_RES1 | OPT_PRE)) == 0,
                 "the tile form computes the default sources with inline cross terms");
   using PR = Pairs<NDIM>;
   using T = S;
@@ -299,16 +370,19 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
 #pragma unroll
       for (int iw = 0; iw < NP; ++iw) acc[iw] = base[iw * sP + cg];
     }
-    T dxv[NDIM];
+    T dxv[NDIM], rxv[NDIM];  // the cell widths and their reciprocals
 #pragma unroll
-    for (int d = 0; d < NDIM; ++d) dxv[d] = (T)__ldg(a.fDX[d] + o.X + cg);
+    for (int d = 0; d < NDIM; ++d) width_at(a, o, d, pos[d], cg, dxv[d], rxv[d]);
+    constexpr T r12 = T(1.0 / 12.0);
     // gradient4 (src/vacgrid.t:684): -(q(+2) - 8(q(+1)-q(-1)) - q(-2))/dx/12, zero on
     // the first and last two mesh cells along its dimension (:690-709)
     bool z4[NDIM];
 #pragma unroll
     for (int d = 0; d < NDIM; ++d) z4[d] = pos[d] <= g.lo[d] + 1 || pos[d] >= g.hi[d] - 1;
-    auto g4 = [&](const S* q, int s, T dxd) {
-      return -(ldt<TILE>(q, c + 2 * s) - T(8) * (ldt<TILE>(q, c + s) - ldt<TILE>(q, c - s)) - ldt<TILE>(q, c - 2 * s)) / dxd / T(12);
+    auto g4 = [&](const S* q, int d) {
+      const int s = st[d];
+      const T n = -(ldt<TILE>(q, c + 2 * s) - T(8) * (ldt<TILE>(q, c + s) - ldt<TILE>(q, c - s)) - ldt<TILE>(q, c - 2 * s));
+      return qdiv<FAST>(qdiv<FAST>(n, dxv[d], rxv[d]), T(12), r12);
     };
     const T qdt = (T)qdt_d;
 
@@ -317,29 +391,31 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
     if constexpr ((OPT & OPT_PART_B) == 0) {
 #pragma unroll
     for (int d = 0; d < NDIM; ++d) {
-      if (d < a.dmin || d > a.dmax) continue;
-      if (!z4[d]) {
+      if (!FAST && (d < a.dmin || d > a.dmax)) continue;
 #pragma unroll
-        for (int iw = 0; iw < NP; ++iw) {
-          if (iw == B0 + 1 + d) continue;  // no flux of b_d along d
-          if (!((a.iwmask >> iw) & 1u)) continue;
-          acc[iw] = acc[iw] - qdt * g4(FF(d, iw), st[d], dxv[d]);
-        }
+      for (int iw = 0; iw < NP; ++iw) {
+        if (!FAST && z4[d]) break;
+        if (iw == B0 + 1 + d) continue;  // no flux of b_d along d
+        if (!FAST && !((a.iwmask >> iw) & 1u)) continue;
+        const T t = acc[iw] - qdt * g4(FF(d, iw), d);
+        acc[iw] = z4[d] ? acc[iw] : t;
       }
-      if ((a.iwmask >> E) & 1u) {
+      if (FAST || ((a.iwmask >> E) & 1u)) {
         const S* vd = Df(1 + d);
-        if (!z4[d]) {
-          // getptotal_bg, src/vacphys0.t.mhd:221
-          double bgs = 0.0;
+        // getptotal_bg, src/vacphys0.t.mhd:221
+        double bgs = 0.0;
 #pragma unroll
-          for (int C = 0; C < NDIR; ++C) bgs = bgs + __ldg(BG(2 + C) + cg) * __ldg(BG(2 + C) + cg);
-          const T fb = (T)((a.gamma - 1.0) * __ldg(BG(0) + cg) - 0.5 * (a.gamma - 2.0) * bgs);
-          acc[E] = acc[E] - qdt * g4(vd, st[d], dxv[d]) * fb;
+        for (int C = 0; C < NDIR; ++C) bgs = bgs + __ldg(BG(2 + C) + cg) * __ldg(BG(2 + C) + cg);
+        const T fb = (T)((a.gamma - 1.0) * __ldg(BG(0) + cg) - 0.5 * (a.gamma - 2.0) * bgs);
+        if (FAST || !z4[d]) {
+          const T t = acc[E] - qdt * g4(vd, d) * fb;
+          acc[E] = z4[d] ? acc[E] : t;
         }
 #pragma unroll
         for (int di = 0; di < NDIM; ++di) {
-          if (di < a.dmin || di > a.dmax || z4[di]) continue;
-          acc[E] = acc[E] + qdt * (T)__ldg(BG(2 + di) + cg) * (T)__ldg(BG(2 + d) + cg) * g4(vd, st[di], dxv[di]);
+          if (!FAST && (di < a.dmin || di > a.dmax || z4[di])) continue;
+          const T t = acc[E] + qdt * (T)__ldg(BG(2 + di) + cg) * (T)__ldg(BG(2 + d) + cg) * g4(vd, di);
+          acc[E] = z4[di] ? acc[E] : t;
         }
       }
     }
@@ -349,9 +425,9 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
       const T rho = ldt<TILE>(W(0), c);
 #pragma unroll
       for (int d = 0; d < NDIM; ++d)
-        if (((a.iwmask >> (1 + d)) & 1u) && fabs(a.grav[d]) > kSmall)
+        if ((FAST || ((a.iwmask >> (1 + d)) & 1u)) && fabs(a.grav[d]) > kSmall)
           acc[1 + d] = acc[1 + d] + q2 * (T)a.grav[d] * rho;
-      if ((a.iwmask >> E) & 1u) {
+      if (FAST || ((a.iwmask >> E) & 1u)) {
         const T rt = ldt<TILE>(Df(0), c);
 #pragma unroll
         for (int d = 0; d < NDIM; ++d)
@@ -363,7 +439,8 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
       S* part = (S*)a.out + o.P;
 #pragma unroll
       for (int iw = 0; iw < NP; ++iw) part[iw * sP + cg] = acc[iw];
-    } else {
+      return;
+    }
 
     // --- hyperdiffusion, src/vacusr.viscosity.t:2-221 --------------------------------
     if (a.visc_on) {
@@ -372,6 +449,8 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
 #pragma unroll
       for (int d = 0; d < NDIM; ++d)
         z1[d] = (a.zero1[d][0] && pos[d] == g.lo[d]) || (a.zero1[d][1] && pos[d] == g.hi[d]);
+      auto over = [&](T n, int d) { return qdiv<FAST>(n, dxv[d], rxv[d]); };
+      auto zero_if = [](bool z, T v) { return z ? T(0) : v; };
       auto nus = [&](int ip, int k, int j, T dxk, T& nl, T& nr) {
         const S* Qp = QQ(ip);
         nr = ldt<TILE>(Qp, j) * dxk;
@@ -388,10 +467,10 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
           nus(pass == 0 ? PR::rho(k) : PR::e(k), k, c, dxv[k], nl, nr);
           numax = fmaxT(numax, fmaxT(nr, nl));
           const T qc = ldt<TILE>(q, c);
-          const T gL = z1[k] ? T(0) : (qc - ldt<TILE>(q, c - st[k])) / dxv[k];
-          const T gR = z1[k] ? T(0) : (ldt<TILE>(q, c + st[k]) - qc) / dxv[k];
+          const T gL = zero_if(z1[k], over(qc - ldt<TILE>(q, c - st[k]), k));
+          const T gR = zero_if(z1[k], over(ldt<TILE>(q, c + st[k]) - qc, k));
           const T tL = (nl + T(0)) * gL, tR = (nr + T(0)) * gR;
-          acc[tgt] = acc[tgt] + (tR - tL) / dxv[k] * q2;
+          acc[tgt] = acc[tgt] + over(tR - tL, k) * q2;
         }
       }
       // momentum, :69-133
@@ -409,14 +488,14 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
           nus(PR::v(l, k), k, c, dxk, nl, nr);
           numax = fmaxT(numax, fmaxT(nr, nl));
           const T qc = ldt<TILE>(q, c);
-          const T gL = z1[k] ? T(0) : (qc - ldt<TILE>(q, c - sk)) / dxk;
-          const T gR = z1[k] ? T(0) : (ldt<TILE>(q, c + sk) - qc) / dxk;
+          const T gL = zero_if(z1[k], over(qc - ldt<TILE>(q, c - sk), k));
+          const T gR = zero_if(z1[k], over(ldt<TILE>(q, c + sk) - qc, k));
           const T tL = (nl + T(0)) * gL, tR = (nr + T(0)) * gR;
           const S* ml = W(1 + l);
           const T mc = ldt<TILE>(ml, c);
           const T VL = (mc + ldt<TILE>(ml, c - sk)) / T(2), VR = (ldt<TILE>(ml, c + sk) + mc) / T(2);
-          const T t2m = (rR * tR - rL * tL) / dxk / T(2);
-          const T t2e = (VR * tR - VL * tL) / dxk / T(2);
+          const T t2m = over(rR * tR - rL * tL, k) / T(2);
+          const T t2e = over(VR * tR - VL * tL, k) / T(2);
           // ii1=0: i=k, ii0=l
           acc[1 + l] = acc[1 + l] + t2m * q2;
           acc[E] = acc[E] + t2e * q2;
@@ -434,23 +513,24 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
               const long jg = sg ? cg + stg[l] : cg - stg[l];
               const int pl = pos[l] + (sg ? 1 : -1);
               T H = T(0);
-              if (pl >= g.lo[l] && pl <= g.hi[l]) {  // nu vanishes outside the mesh
-                if constexpr ((OPT & OPT_PRE) != 0) {
-                  H = ldt<TILE>((const S*)a.fX[Cross<NDIM>::m(l, k)] + o.I, j);
-                } else {
-                  const T dxkj = (T)__ldg(a.fDX[k] + o.X + jg);
+              const bool in = pl >= g.lo[l] && pl <= g.hi[l];  // nu vanishes outside the mesh
+              if constexpr ((OPT & OPT_PRE) != 0) {
+                H = zero_if(!in, ldt<TILE>((const S*)a.fX[Cross<NDIM>::m(l, k)] + o.I, j));
+              } else {
+                if (in) {
+                  T dxkj, rxkj;
+                  width_at(a, o, k, pos[k], jg, dxkj, rxkj);
                   T njl, njr;
                   nus(PR::v(l, k), k, j, dxkj, njl, njr);
-                  const T gC = z1[k] ? T(0) : (ldt<TILE>(q, j + sk) - ldt<TILE>(q, j - sk)) / dxkj / T(2);
+                  const T gC = z1[k] ? T(0) : qdiv<FAST>(ldt<TILE>(q, j + sk) - ldt<TILE>(q, j - sk), dxkj, rxkj) / T(2);
                   H = gC * (njl + njr + T(2) * T(0)) / T(2) / T(2);
                 }
               }
               Tm[sg] = ldt<TILE>(rtf, j) * H;
               Te[sg] = ldt<TILE>(W(1 + k), j) * H;
             }
-            const T dxl = dxv[l];
-            const T tCm = z1[l] ? T(0) : (Tm[1] - Tm[0]) / dxl / T(2);
-            const T tCe = z1[l] ? T(0) : (Te[1] - Te[0]) / dxl / T(2);
+            const T tCm = zero_if(z1[l], over(Tm[1] - Tm[0], l) / T(2));
+            const T tCe = zero_if(z1[l], over(Te[1] - Te[0], l) / T(2));
             acc[1 + k] = acc[1 + k] + tCm * q2;
             acc[E] = acc[E] + tCe * q2;
           }
@@ -477,23 +557,24 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
               const long jg = sg ? cg + stg[l] : cg - stg[l];
               const int pl = pos[l] + (sg ? 1 : -1);
               T Kv = T(0);
-              if (pl >= g.lo[l] && pl <= g.hi[l]) {
-                if constexpr ((OPT & OPT_PRE) != 0) {
-                  Kv = ldt<TILE>((const S*)a.fX[Cross<NDIM>::b(l, k)] + o.I, j);
-                } else {
-                  const T dxkj = (T)__ldg(a.fDX[k] + o.X + jg);
+              const bool in = pl >= g.lo[l] && pl <= g.hi[l];
+              if constexpr ((OPT & OPT_PRE) != 0) {
+                Kv = zero_if(!in, ldt<TILE>((const S*)a.fX[Cross<NDIM>::b(l, k)] + o.I, j));
+              } else {
+                if (in) {
+                  T dxkj, rxkj;
+                  width_at(a, o, k, pos[k], jg, dxkj, rxkj);
                   T njl, njr;
                   nus(PR::b(l, k), k, j, dxkj, njl, njr);
-                  const T gC = z1[k] ? T(0) : (ldt<TILE>(q, j + sk) - ldt<TILE>(q, j - sk)) / dxkj / T(2);
+                  const T gC = z1[k] ? T(0) : qdiv<FAST>(ldt<TILE>(q, j + sk) - ldt<TILE>(q, j - sk), dxkj, rxkj) / T(2);
                   Kv = gC * (njl + njr) / T(2);
                 }
               }
               K[sg] = Kv;
               Ke[sg] = Kv * ldt<TILE>(W(B0 + 1 + k), j);
             }
-            const T dxl = dxv[l];
-            const T tC = z1[l] ? T(0) : (K[1] - K[0]) / dxl / T(2);
-            const T tCe = z1[l] ? T(0) : (Ke[1] - Ke[0]) / dxl / T(2);
+            const T tC = zero_if(z1[l], over(K[1] - K[0], l) / T(2));
+            const T tCe = zero_if(z1[l], over(Ke[1] - Ke[0], l) / T(2));
             acc[B0 + 1 + k] = acc[B0 + 1 + k] + T(-1) * tC * q2;
             acc[E] = acc[E] + T(-1) * tCe * q2;
           }
@@ -501,11 +582,11 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
           {
             const T qc = ldt<TILE>(q, c), qm = ldt<TILE>(q, c - sk), qp = ldt<TILE>(q, c + sk);
             const T BL = (qc + qm) / T(2), BR = (qp + qc) / T(2);
-            const T gL = z1[k] ? T(0) : (qc - qm) / dxk;
-            const T gR = z1[k] ? T(0) : (qp - qc) / dxk;
+            const T gL = zero_if(z1[k], over(qc - qm, k));
+            const T gR = zero_if(z1[k], over(qp - qc, k));
             const T tL = nl * gL, tR = nr * gR;
-            acc[B0 + 1 + l] = acc[B0 + 1 + l] + T(1) * (tR - tL) / dxk * q2;
-            acc[E] = acc[E] + T(1) * (tR * BR - tL * BL) / dxk * q2;
+            acc[B0 + 1 + l] = acc[B0 + 1 + l] + over(T(1) * (tR - tL), k) * q2;
+            acc[E] = acc[E] + over(T(1) * (tR * BR - tL * BL), k) * q2;
           }
         }
     }
@@ -543,7 +624,9 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
     // direction d outermost keeps the reference's order of additions: d is jdir of
     // the b loop and idir of the e loop.
     constexpr int IDM = res_idirmin(NDIM, NDIR);
-    auto curr = [&](int n, T J[3]) {
+    // J at cell n, which lies sg cells along dimension d from this one
+    auto curr = [&](int n, int d, int sg, T J[3]) {
+      const bool ghost = pos[d] + sg < g.lo[d] || pos[d] + sg > g.hi[d];
 #pragma unroll
       for (int i = IDM; i < 3; ++i) {
         J[i] = T(0);
@@ -554,8 +637,10 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
             const int l = lvc3(i, j, k);
             if (l == 0) continue;
             const int sj = st[j];
-            const T dxn = (T)__ldg(a.fDX[j] + o.X + n);
-            const T gr = -(Bat(k, n + sj) - Bat(k, n - sj)) / dxn / T(2);
+            T dxn, rxn;
+            const int row = (j != d && ghost) ? 1 + 2 * (d < j ? d : d - 1) + (sg > 0 ? 1 : 0) : 0;
+            width_at(a, o, j, row * g.n[j] + pos[j] + (j == d ? sg : 0), (long)n, dxn, rxn);
+            const T gr = qdiv<FAST>(-(Bat(k, n + sj) - Bat(k, n - sj)), dxn, rxn) / T(2);
             J[i] = (l == 1) ? J[i] + gr : J[i] - gr;
           }
       }
@@ -567,21 +652,20 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
         for (int d = 0; d < NDIM; ++d) {
           const int s = st[d];
           T Jp[3], Jm[3];
-          curr(c + s, Jp);
-          curr(c - s, Jm);
-          const T dxd = dxv[d];
+          curr(c + s, d, 1, Jp);
+          curr(c - s, d, -1, Jm);
 #pragma unroll
           for (int i = 0; i < NDIR; ++i) {
-            if (!((a.iwmask >> (B0 + 1 + i)) & 1u)) continue;
+            if (!FAST && !((a.iwmask >> (B0 + 1 + i)) & 1u)) continue;
 #pragma unroll
             for (int k = IDM; k < 3; ++k) {
               const int l = lvc3(i, d, k);
               if (l == 0) continue;
-              const T gr = -(Jp[k] * eta * q2 - Jm[k] * eta * q2) / dxd / T(2);
+              const T gr = qdiv<FAST>(-(Jp[k] * eta * q2 - Jm[k] * eta * q2), dxv[d], rxv[d]) / T(2);
               acc[B0 + 1 + i] = (l == 1) ? acc[B0 + 1 + i] - gr : acc[B0 + 1 + i] + gr;
             }
           }
-          if ((a.iwmask >> E) & 1u) {
+          if (FAST || ((a.iwmask >> E) & 1u)) {
 #pragma unroll
             for (int j = 0; j < NDIR; ++j) {
 #pragma unroll
@@ -589,7 +673,7 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
                 const int l = lvc3(d, j, k);
                 if (l == 0) continue;
                 const T up = Bat(j, c + s) * Jp[k] * eta * q2, um = Bat(j, c - s) * Jm[k] * eta * q2;
-                const T gr = -(up - um) / dxd / T(2);
+                const T gr = qdiv<FAST>(-(up - um), dxv[d], rxv[d]) / T(2);
                 acc[E] = (l == 1) ? acc[E] + gr : acc[E] - gr;
               }
             }
@@ -615,13 +699,13 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
           lap = lap + (Bat(i, c + s) - T(2) * Bc + Bat(i, c - s)) / (dxd * dxd);
         }
         lap = lap * eta;
-        if ((a.iwmask >> (B0 + 1 + i)) & 1u) acc[B0 + 1 + i] = acc[B0 + 1 + i] + q2 * lap;
-        if ((a.iwmask >> E) & 1u) acc[E] = acc[E] + q2 * lap * Bc;
+        if (FAST || ((a.iwmask >> (B0 + 1 + i)) & 1u)) acc[B0 + 1 + i] = acc[B0 + 1 + i] + q2 * lap;
+        if (FAST || ((a.iwmask >> E) & 1u)) acc[E] = acc[E] + q2 * lap * Bc;
       }
       if constexpr (IDM < 3) {
-        if ((a.iwmask >> E) & 1u) {
+        if (FAST || ((a.iwmask >> E) & 1u)) {
           T J[3];
-          curr(c, J);
+          curr(c, 0, 0, J);
           T j2 = T(0);
 #pragma unroll
           for (int i = IDM; i < 3; ++i) j2 = j2 + J[i] * J[i];
@@ -636,11 +720,9 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
       T divb = T(0);
 #pragma unroll
       for (int d = 0; d < NDIM; ++d) {
-        T gd = T(0);
-        if (!z4[d]) {
-          const int s = st[d];
-          gd = -(Bat(d, c + 2 * s) - T(8) * (Bat(d, c + s) - Bat(d, c - s)) - Bat(d, c - 2 * s)) / dxv[d] / T(12);
-        }
+        const int s = st[d];
+        const T n4 = -(Bat(d, c + 2 * s) - T(8) * (Bat(d, c + s) - Bat(d, c - s)) - Bat(d, c - 2 * s));
+        const T gd = z4[d] ? T(0) : qdiv<FAST>(qdiv<FAST>(n4, dxv[d], rxv[d]), T(12), r12);
         divb = divb + gd;
       }
       divb = q2 * divb;
@@ -650,11 +732,11 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
       for (int C = 0; C < NDIR; ++C) {
         const T mC = ldt<TILE>(W(1 + C), c);
         const T BC = Bat(C, c);
-        if ((a.iwmask >> (1 + C)) & 1u) acc[1 + C] = acc[1 + C] - BC * divb;
-        if ((a.iwmask >> (B0 + 1 + C)) & 1u) acc[B0 + 1 + C] = acc[B0 + 1 + C] - mC / rt * divb;
+        if (FAST || ((a.iwmask >> (1 + C)) & 1u)) acc[1 + C] = acc[1 + C] - BC * divb;
+        if (FAST || ((a.iwmask >> (B0 + 1 + C)) & 1u)) acc[B0 + 1 + C] = acc[B0 + 1 + C] - ldt<TILE>(Df(1 + C), c) * divb;
         sm = (C == 0) ? mC * BC : sm + mC * BC;
       }
-      if ((a.iwmask >> E) & 1u) acc[E] = acc[E] - sm / rt * divb;
+      if (FAST || ((a.iwmask >> E) & 1u)) acc[E] = acc[E] - sm / rt * divb;
     }
 
     // --- store with the Runge-Kutta epilogue (src/vac.t:450,454) ---------------------
@@ -676,9 +758,7 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
 #pragma unroll
       for (int iw = 0; iw < NP; ++iw) out[iw * sP + cg] = acc[iw] + w1[iw * sP + cg];
     }
-
-    }  // part B
-    }
+  }
   numax_out = fmax(numax_out, (double)numax);
 }
 
@@ -686,9 +766,9 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
 // single-grid kernels
 // ---------------------------------------------------------------------------
 // resident blocks per SM of the face and setnu passes (measured at 128^3, like
-// the update's below: face 1.11 -> 0.82 ms in FP64 at 4 blocks, nu 1.04 -> 0.98
-// ms in FP64 at 6; FP32 setnu is fastest at the 80 registers of 3 blocks, which
-// the compiler chose without a bound until the argument struct grew)
+// the update's below: face 124 us per launch in FP64 at 4 blocks, 146 at 2, 161 at 5;
+// nu 204 us in FP64 at 6; FP32 face 81 us at 4, 102 at 3; FP32 setnu is fastest at the
+// 80 registers of 3 blocks)
 #ifndef SAC_FACE_MINB_F64
 #define SAC_FACE_MINB_F64 4
 #endif
@@ -711,11 +791,36 @@ __global__ void __launch_bounds__(256, sizeof(S) == 8 ? SAC_FACE_MINB_F64 : SAC_
   double cm[NDIM];
 #pragma unroll
   for (int d = 0; d < NDIM; ++d) cm[d] = 0.0;
+  bool bad = false;
+  const bool sampled = blockIdx.x % 16 == 0;  // a.nbad counts one block in 16, which is enough for its use
+  const int p0 = c % g.n[0], p1 = (c / g.n[0]) % g.n[1], p2 = c / (g.n[0] * g.n[1]);
   if (c < (int)g.ncell) {
-    const int p0 = c % g.n[0], p1 = (c / g.n[0]) % g.n[1], p2 = c / (g.n[0] * g.n[1]);
     const bool mesh = do_ctot && p0 >= g.lo[0] && p0 <= g.hi[0] && p1 >= g.lo[1] && p1 <= g.hi[1] &&
                       p2 >= g.lo[2] && p2 <= g.hi[2];
-    face_cell<NDIM, NDIR, S>(a, Offs{0, 0, 0, 0}, c, mesh, a.gamma, cm);
+    bad = face_cell<NDIM, NDIR, S>(a, Offs{}, c, mesh, a.gamma, cm, sampled || !a.quiet);
+  }
+  if constexpr (sizeof(S) == 8) {
+    // flag the bricks around each brick in which this warp has a cell out of range (a
+    // stencil reaches 3 cells): one lane per neighbour
+    const unsigned all = __ballot_sync(0xffffffffu, bad);
+    const int lane = threadIdx.x & 31;
+    if (all && !a.quiet) {  // the quiet form's kernels read no flags
+      const int brick = (p0 >> 3) + a.fst[1] * (p1 >> 3) + a.fst[2] * (p2 >> 3);
+      const int before = __shfl_up_sync(0xffffffffu, brick, 1);
+      const bool leads = bad && !(lane > 0 && ((all >> (lane - 1)) & 1u) && before == brick);
+      for (unsigned m = __ballot_sync(0xffffffffu, leads); m; m &= m - 1) {
+        const int src = __ffs(m) - 1;
+        const int b0 = (__shfl_sync(0xffffffffu, p0, src) >> 3) + lane % 3 - 1;
+        const int b1 = (__shfl_sync(0xffffffffu, p1, src) >> 3) + (lane / 3) % 3 - 1;
+        const int b2 = (__shfl_sync(0xffffffffu, p2, src) >> 3) + lane / 9 - 1;
+        if (lane < 27 && b0 >= 0 && b0 <= (g.n[0] - 1) >> 3 && b1 >= 0 && b1 <= (g.n[1] - 1) >> 3 && b2 >= 0 &&
+            b2 <= (g.n[2] - 1) >> 3) {
+          unsigned char* f = a.flags + b0 + a.fst[1] * b1 + a.fst[2] * b2;
+          if (!__ldcg(f)) *f = 1;  // most are set: reads of a hot sector do not queue as writes do
+        }
+      }
+    }
+    if (NDIM == 3 && all && sampled && lane == 0) atomicAdd(a.nbad, 16u * (unsigned)__popc(all));
   }
   if (do_ctot) {
 #pragma unroll
@@ -738,14 +843,29 @@ __global__ void __launch_bounds__(256, sizeof(S) == 8 ? SAC_NU_MINB_F64 : SAC_NU
 #pragma unroll
   for (int d = 0; d < 3; ++d) p[d] += (d < NDIM) ? g.lo[d] - 1 : 0;
   const int c = p[0] + (int)g.st[1] * p[1] + (int)g.st[2] * p[2];
-  nu_cell<NDIM, NDIR, S>(a, g, Offs{0, 0, 0, 0}, c, p, a.ctot);
+  nu_cell<NDIM, NDIR, S>(a, g, Offs{}, c, p, a.ctot);
+}
+
+// Whether the cells of this warp take the general form (FAST = false): the launch
+// does, or in FP64 a brick that one of them lies in is flagged or setnu's c_tot is out
+// of range (in: this thread has a mesh cell, at pos)
+template <int NDIM, typename S>
+__device__ __forceinline__ bool takes_divide(const Stage2Args& a, bool in, const int pos[3]) {
+  bool slow = a.general || a.quiet;
+  if constexpr (sizeof(S) != 8) return slow;
+  if (a.visc_on) {
+#pragma unroll
+    for (int d = 0; d < NDIM; ++d) slow = slow || ctot_out_of_range(a.ctot[d]);
+  }
+  if (in) slow = slow || __ldg(a.flags + (pos[0] >> 3) + a.fst[1] * (pos[1] >> 3) + a.fst[2] * (pos[2] >> 3)) != 0;
+  return __any_sync(0xffffffffu, slow);
 }
 
 // k_cross body at the mesh cell pos: for every l != k the centred half-sums of
 // addsource_visc's cross derivatives at this cell, which the update of the cells
 // on either side along l uses (src/vacusr.viscosity.t:117-118 for the momenta,
 // :195-197 for the field) -- the same expressions as the update's inline form
-template <int NDIM, int NDIR, typename S>
+template <int NDIM, int NDIR, typename S, bool FAST>
 __device__ __forceinline__ void cross_cell(const Stage2Args& a, const Geom& g, const Offs& o, const int pos[3]) {
   using PR = Pairs<NDIM>;
   using CR = Cross<NDIM>;
@@ -757,7 +877,8 @@ __device__ __forceinline__ void cross_cell(const Stage2Args& a, const Geom& g, c
   for (int k = 0; k < NDIM; ++k) {
     const int sk = st[k];
     const bool z1 = (a.zero1[k][0] && pos[k] == g.lo[k]) || (a.zero1[k][1] && pos[k] == g.hi[k]);
-    const T dxk = (T)__ldg(a.fDX[k] + o.X + c);
+    T dxk, rxk;
+    width_at(a, o, k, pos[k], (long)c, dxk, rxk);
 #pragma unroll
     for (int l = 0; l < NDIM; ++l) {
       if (l == k) continue;
@@ -765,24 +886,26 @@ __device__ __forceinline__ void cross_cell(const Stage2Args& a, const Geom& g, c
         const S* q = (const S*)a.fD[1 + l] + o.I;
         const S* Qp = (const S*)a.fQ[PR::v(l, k)] + o.I;
         const T nr = ld(Qp, c) * dxk, nl = ld(Qp, c - sk) * dxk;
-        const T gC = z1 ? T(0) : (ld(q, c + sk) - ld(q, c - sk)) / dxk / T(2);
+        const T g1 = qdiv<FAST>(ld(q, c + sk) - ld(q, c - sk), dxk, rxk) / T(2);
+        const T gC = z1 ? T(0) : g1;
         ((S*)a.fX[CR::m(l, k)] + o.I)[c] = gC * (nl + nr + T(2) * T(0)) / T(2) / T(2);
       }
       {  // field: b_l along k
         const S* q = (const S*)a.fW[B0 + 1 + l] + o.P;
         const S* Qp = (const S*)a.fQ[PR::b(l, k)] + o.I;
         const T nr = ld(Qp, c) * dxk, nl = ld(Qp, c - sk) * dxk;
-        const T gC = z1 ? T(0) : (ld(q, c + sk) - ld(q, c - sk)) / dxk / T(2);
+        const T g1 = qdiv<FAST>(ld(q, c + sk) - ld(q, c - sk), dxk, rxk) / T(2);
+        const T gC = z1 ? T(0) : g1;
         ((S*)a.fX[CR::b(l, k)] + o.I)[c] = gC * (nl + nr) / T(2);
       }
     }
   }
 }
 
-// 8 resident blocks per SM (32 registers): measured at 128^3 in FP64, setnu plus
-// k_cross 1.565 -> 1.499 ms per RK4 step against the unbounded 44 registers
+// 6 resident blocks per SM: measured in FP64 103.6 us per launch at 128^3 (108 at 8
+// and 107 at 5) and 3.5 us at 251x187 (4.1 at 8)
 #ifndef SAC_CROSS_MINB
-#define SAC_CROSS_MINB 8
+#define SAC_CROSS_MINB 6
 #endif
 template <int NDIM, int NDIR, typename S>
 __global__ void __launch_bounds__(256, SAC_CROSS_MINB) k_cross(const Stage2Args a) {
@@ -791,66 +914,30 @@ __global__ void __launch_bounds__(256, SAC_CROSS_MINB) k_cross(const Stage2Args 
   pos[0] = g.lo[0] + blockIdx.x * blockDim.x + threadIdx.x;
   pos[1] = g.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
   pos[2] = g.lo[2] + blockIdx.z * blockDim.z + threadIdx.z;
-  if (pos[0] <= g.hi[0] && pos[1] <= g.hi[1] && pos[2] <= g.hi[2])
-    cross_cell<NDIM, NDIR, S>(a, g, Offs{0, 0, 0, 0}, pos);
+  const bool in = pos[0] <= g.hi[0] && pos[1] <= g.hi[1] && pos[2] <= g.hi[2];
+  const bool slow = takes_divide<NDIM, S>(a, in, pos);
+  if (!in) return;
+  if (slow)
+    cross_cell<NDIM, NDIR, S, false>(a, g, Offs{}, pos);
+  else
+    cross_cell<NDIM, NDIR, S, true>(a, g, Offs{}, pos);
 }
 
-// Resident blocks of 256 threads per SM that the register budget is sized for.
-// The update is latency-bound; filling more warp slots beats keeping every
-// value in registers (measured at 128^3: FP64 1.91 -> 1.55 ms per launch going
-// from 2 to 4 blocks, FP32 0.95 -> 0.53 ms going from 2 to 8, the extra spills
-// served from L1).
-#ifndef SAC_UPDATE_MINB_F64
-#define SAC_UPDATE_MINB_F64 4
-#endif
-#ifndef SAC_UPDATE_MINB_F32
-#define SAC_UPDATE_MINB_F32 8
-#endif
-
-// the 3D update's block shape per storage type (256 threads; x along the
-// contiguous dimension)
-#ifndef SAC_UPDATE_BLK3_F64_X
-#define SAC_UPDATE_BLK3_F64_X 8
-#define SAC_UPDATE_BLK3_F64_Y 8
-#define SAC_UPDATE_BLK3_F64_Z 4
-#endif
-#ifndef SAC_UPDATE_BLK3_F32_X
-#define SAC_UPDATE_BLK3_F32_X 32
-#define SAC_UPDATE_BLK3_F32_Y 4
-#define SAC_UPDATE_BLK3_F32_Z 2
-#endif
-
-// The FP64 3D update runs in two parts (bit 0; bit 1 would split the FP32 one):
-// part A (centdiff4 and gravity) needs fewer registers and runs at 5 resident
-// blocks per SM without spills, part B (hyperdiffusion to the epilogue) at 4.
-// Measured at 128^3 on one B200, same box: 2.92e8 -> 3.00e8 FP64 cell-updates/s
-// (update 4.47 -> 4.27 ms per step); at 4 blocks for both parts no gain; the
-// FP32 update split at 8 / 6 blocks is 1 % slower and stays whole.
-#ifndef SAC_UPDATE_SPLIT
-#define SAC_UPDATE_SPLIT 1
-#endif
-#ifndef SAC_UPDATE_A_MINB_F64
-#define SAC_UPDATE_A_MINB_F64 5
-#endif
-#ifndef SAC_UPDATE_B_MINB_F64
-#define SAC_UPDATE_B_MINB_F64 4
-#endif
-#ifndef SAC_UPDATE_A_MINB_F32
-#define SAC_UPDATE_A_MINB_F32 8
-#endif
-#ifndef SAC_UPDATE_B_MINB_F32
-#define SAC_UPDATE_B_MINB_F32 8
-#endif
-template <typename S, int OPT>
+// Resident blocks of 256 threads per SM that the register budget is sized for.  With
+// its loads free of branches the compiler issues them in groups as far as the
+// registers reach, which beats more warps whose values spill: measured at 128^3 in
+// FP64 (random modes) 681 us per launch at 2 blocks, 778 at 3, against 961 for the
+// two launches at 5 and 4 blocks before; FP32 298 us at 4, 308 at 3, 421 at 5, 511 at
+// 8.  The plain 2D update fits in fewer: FP64 at 512^2 31.3 us at 4 blocks, 35.2 at 3,
+// 39 at 2; with the Powell and resistive terms (251x187) 11.3 us at 2, 15.4 at 4.
+template <typename S, int NDIM, int OPT>
 constexpr int update_minb() {
-  return sizeof(S) != 8 ? ((OPT & OPT_PART_A) ? SAC_UPDATE_A_MINB_F32
-                                              : ((OPT & OPT_PART_B) ? SAC_UPDATE_B_MINB_F32 : SAC_UPDATE_MINB_F32))
-                        : ((OPT & OPT_PART_A) ? SAC_UPDATE_A_MINB_F64
-                                              : ((OPT & OPT_PART_B) ? SAC_UPDATE_B_MINB_F64 : SAC_UPDATE_MINB_F64));
+  if (OPT & OPT_QUIET) return (OPT & OPT_PART_A) ? 5 : 4;
+  return sizeof(S) == 8 ? (NDIM == 2 && (OPT & ~OPT_PRE) == 0 ? 4 : 2) : 4;
 }
 
 template <int NDIM, int NDIR, typename S, int OPT>
-__global__ void __launch_bounds__(256, update_minb<S, OPT>())
+__global__ void __launch_bounds__(256, update_minb<S, NDIM, OPT>())
     k_update(const Stage2Args a) {
   __shared__ double sh[32];
   const Geom& g = a.g;
@@ -859,11 +946,20 @@ __global__ void __launch_bounds__(256, update_minb<S, OPT>())
   pos[1] = g.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
   pos[2] = g.lo[2] + blockIdx.z * blockDim.z + threadIdx.z;
   double numax = 0.0;
-  if (pos[0] <= g.hi[0] && pos[1] <= g.hi[1] && pos[2] <= g.hi[2])
-    update_cell<NDIM, NDIR, S, OPT>(a, g, Offs{0, 0, 0, 0}, pos, a.qdt, a.qdt2, a.tdep, a.drvA, numax);
-  if constexpr ((OPT & OPT_PART_A) == 0) {
-    if (a.visc_on) block_max_to(a.maxnu, numax, sh);
+  const bool in = pos[0] <= g.hi[0] && pos[1] <= g.hi[1] && pos[2] <= g.hi[2];
+  if constexpr ((OPT & OPT_QUIET) != 0) {
+    if (in) update_cell<NDIM, NDIR, S, OPT, false>(a, g, Offs{}, pos, a.qdt, a.qdt2, a.tdep, a.drvA, numax);
+    if constexpr ((OPT & OPT_PART_A) != 0) return;
+  } else {
+    const bool slow = takes_divide<NDIM, S>(a, in, pos);
+    if (in) {
+      if (slow)
+        update_cell<NDIM, NDIR, S, OPT, false>(a, g, Offs{}, pos, a.qdt, a.qdt2, a.tdep, a.drvA, numax);
+      else
+        update_cell<NDIM, NDIR, S, OPT, true>(a, g, Offs{}, pos, a.qdt, a.qdt2, a.tdep, a.drvA, numax);
+    }
   }
+  if (a.visc_on) block_max_to(a.maxnu, numax, sh);
 }
 
 // ---------------------------------------------------------------------------
@@ -951,7 +1047,7 @@ __global__ void __launch_bounds__(256, sizeof(S) == 8 ? SAC_BATCH_UPDATE_MINB_F6
       const double qdt = b.stage == 0 ? dt / 2 : b.stage == 1 ? dt / 2 : b.stage == 2 ? dt : dt / 6;
       const double qdt2 = qdt * ((double)(b.a.dmax - b.a.dmin) + 1.0) / (double)g.ndim;
       const double tdep = b.a.driver != DRV_NONE ? sin(omega * tnow) : 0.0;
-      update_cell<NDIM, NDIR, S, OPT>(b.a, g, I.o, p, qdt, qdt2, tdep, drvA, numax);
+      update_cell<NDIM, NDIR, S, OPT, sizeof(S) != 8>(b.a, g, I.o, p, qdt, qdt2, tdep, drvA, numax);
     }
     if (b.a.visc_on) block_max_to(&b.dyn[tl.inst].maxnu, numax, sh);
   }
@@ -999,7 +1095,7 @@ __device__ __forceinline__ void courant_tile(const BatchStageArgs& b, int t, dou
       for (int d = 0; d < NDIM; ++d) {
         const double Bd = W(E + 1 + d) + BG(2 + d);
         const double cmax = sqrt(0.5 * (cf2 + sqrt(cf2 * cf2 - 4.0 * cs2 * (Bd * Bd) / rt))) + fabs(W(1 + d) / rt);
-        const double r = cmax / b.a.fDX[d][I.o.X + c];
+        const double r = cmax / b.a.dx[d][I.o.X + c];
         best = (r != r) ? r : fmax(best, r);
       }
     }
@@ -1055,10 +1151,7 @@ void launch_update(const Stage2Args& a0, cudaStream_t st) {
   const Geom& g = a.g;
   dispatch_nd(g, [&](auto ND, auto NR) {
     constexpr int NDIM = decltype(ND)::value;
-    dim3 blk = NDIM == 1 ? dim3(256, 1, 1)
-                         : (NDIM == 2 ? dim3(32, 8, 1)
-                                      : (sizeof(S) == 8 ? dim3(SAC_UPDATE_BLK3_F64_X, SAC_UPDATE_BLK3_F64_Y, SAC_UPDATE_BLK3_F64_Z)
-                                                        : dim3(SAC_UPDATE_BLK3_F32_X, SAC_UPDATE_BLK3_F32_Y, SAC_UPDATE_BLK3_F32_Z)));
+    const dim3 blk = NDIM == 1 ? dim3(256, 1, 1) : dim3(32, 8, 1);
     const int n0 = g.hi[0] - g.lo[0] + 1, n1 = g.hi[1] - g.lo[1] + 1, n2 = g.hi[2] - g.lo[2] + 1;
     dim3 grd((n0 + blk.x - 1) / blk.x, (n1 + blk.y - 1) / blk.y, (n2 + blk.z - 1) / blk.z);
     constexpr int NDIR = decltype(NR)::value;
@@ -1066,43 +1159,41 @@ void launch_update(const Stage2Args& a0, cudaStream_t st) {
     // resistive one a current component (ndir > 1)
     const int ropt = a.res_on ? (a.res_compact ? OPT_RES1 : (NDIR > 1 ? OPT_RES : 0)) : 0;
     const int opt = ((NDIM > 1 && a.divb_on) ? OPT_DIVB : 0) | ropt;
-    // the FP64 single grid takes the precomputed cross terms (k_cross runs
-    // whenever hyperdiffusion does; without it the terms are never reached):
-    // measured at 128^3 the update fell from 5.53 to 4.41 ms per step for 0.59
-    // ms of k_cross.  The FP32 update, held to 32 registers, was slower with
-    // them (2.11 -> 2.39 ms) and computes them inline.
-    constexpr int P = sizeof(S) == 8 ? OPT_PRE : 0;
+    // the single grid takes the precomputed cross terms (k_cross runs whenever
+    // hyperdiffusion does; without it the terms are never reached): at 128^3 in FP64
+    // they took 1.1 ms per step off the update for 0.43 ms of k_cross; in FP32 the
+    // update falls from 521 us (inline, 32 registers) to 298 for 68 us of k_cross
+    constexpr int P = OPT_PRE;
+    // a state with many cells out of range (a.quiet): the general form for all of it,
+    // in two launches at 5 and 4 blocks per SM.  At 128^3 from rest 6.6 ms per step so,
+    // 11 in the common kernel, whose registers leave its divides 16 warps per SM
+    auto go = [&](auto o) {
+      constexpr int O = P | decltype(o)::value;
+      if constexpr (NDIM == 3 && sizeof(S) == 8) {
+        if (a.quiet) {
+          const dim3 qblk(8, 8, 4);  // part B 729 us per launch so, 764 at 32x8x1
+          const dim3 qgrd((n0 + qblk.x - 1) / qblk.x, (n1 + qblk.y - 1) / qblk.y, (n2 + qblk.z - 1) / qblk.z);
+          if constexpr (O == P) {
+            k_update<NDIM, NDIR, S, O | OPT_QUIET | OPT_PART_A><<<qgrd, qblk, 0, st>>>(a);
+            k_update<NDIM, NDIR, S, O | OPT_QUIET | OPT_PART_B><<<qgrd, qblk, 0, st>>>(a);
+          } else {
+            k_update<NDIM, NDIR, S, O | OPT_QUIET><<<qgrd, qblk, 0, st>>>(a);
+          }
+          return;
+        }
+      }
+      k_update<NDIM, NDIR, S, O><<<grd, blk, 0, st>>>(a);
+    };
     if constexpr (NDIM > 1) {
-      if (opt == OPT_DIVB) {
-        k_update<NDIM, NDIR, S, P | OPT_DIVB><<<grd, blk, 0, st>>>(a);
-        return;
-      }
-      if (opt == (OPT_DIVB | OPT_RES)) {
-        k_update<NDIM, NDIR, S, P | OPT_DIVB | OPT_RES><<<grd, blk, 0, st>>>(a);
-        return;
-      }
-      if (opt == (OPT_DIVB | OPT_RES1)) {
-        k_update<NDIM, NDIR, S, P | OPT_DIVB | OPT_RES1><<<grd, blk, 0, st>>>(a);
-        return;
-      }
+      if (opt == OPT_DIVB) return go(std::integral_constant<int, OPT_DIVB>{});
+      if (opt == (OPT_DIVB | OPT_RES)) return go(std::integral_constant<int, OPT_DIVB | OPT_RES>{});
+      if (opt == (OPT_DIVB | OPT_RES1)) return go(std::integral_constant<int, OPT_DIVB | OPT_RES1>{});
     }
     if constexpr (NDIR > 1) {
-      if (opt == OPT_RES) {
-        k_update<NDIM, NDIR, S, P | OPT_RES><<<grd, blk, 0, st>>>(a);
-        return;
-      }
+      if (opt == OPT_RES) return go(std::integral_constant<int, OPT_RES>{});
     }
-    if (opt == OPT_RES1) {
-      k_update<NDIM, NDIR, S, P | OPT_RES1><<<grd, blk, 0, st>>>(a);
-      return;
-    }
-    // SAC_UPDATE_SPLIT bit 0: the FP64 3D update in two parts; bit 1: the FP32 one
-    if constexpr (NDIM == 3 && (SAC_UPDATE_SPLIT & (sizeof(S) == 8 ? 1 : 2)) != 0) {
-      k_update<NDIM, NDIR, S, P | OPT_PART_A><<<grd, blk, 0, st>>>(a);
-      k_update<NDIM, NDIR, S, P | OPT_PART_B><<<grd, blk, 0, st>>>(a);
-      return;
-    }
-    k_update<NDIM, NDIR, S, P><<<grd, blk, 0, st>>>(a);
+    if (opt == OPT_RES1) return go(std::integral_constant<int, OPT_RES1>{});
+    go(std::integral_constant<int, 0>{});
   });
 }
 
@@ -1111,7 +1202,7 @@ void launch_cross(const Stage2Args& a0, cudaStream_t st) {
   Stage2Args a = a0;
   fill_field_ptrs(a, sizeof(S));
   const Geom& g = a.g;
-  if (g.ndim < 2 || sizeof(S) != 8) return;  // no pair l != k; FP32 computes them inline
+  if (g.ndim < 2) return;  // no pair l != k
   dispatch_nd(g, [&](auto ND, auto NR) {
     constexpr int NDIM = decltype(ND)::value;
     if constexpr (NDIM > 1) {

@@ -68,7 +68,7 @@ __device__ __forceinline__ void ctot_tile(const BatchStageArgs& b, int t, double
     for (int d = 0; d < NDIM; ++d) cm[d] = 0.0;
     if (tile_cell(tl, g, g.lo, g.hi, p)) {
       const long c = p[0] + g.st[1] * p[1] + g.st[2] * p[2];
-      face_eval<NDIM, NDIR, S>(b.a, I.o, c, true, gamma, cm, 0u, [](int, S) {}, [](int, int, S) {});
+      face_eval<NDIM, NDIR, S>(b.a, I.o, c, true, gamma, cm, 0u, true, [](int, S) {}, [](int, int, S) {});
     }
 #pragma unroll
     for (int d = 0; d < NDIM; ++d) block_max_to(&b.dyn[tl.inst].ctot[d], cm[d], sh);
@@ -100,6 +100,7 @@ __device__ __forceinline__ void stage2d_tile(const BatchStageArgs& b, int t, uns
     const int x0 = tl.p[0], y0 = tl.p[1];  // the tile's first mesh cell
     __syncthreads();  // the previous tile's readers are done with the tile memory
     // ---- phase 1: point fields and fluxes --------------------------------------
+    bool bad = false;  // a box cell's fields are out of qdiv's range
     for (int idx = tid; idx < BW * BH; idx += NT) {
       const int by = idx / BW, bx = idx - by * BW;
       const int gx = x0 - H + bx, gy = y0 - H + by;
@@ -108,8 +109,8 @@ __device__ __forceinline__ void stage2d_tile(const BatchStageArgs& b, int t, uns
       const unsigned fd = ((by >= L::FX_R0 && by < L::FX_R0 + L::FX_NR && bx >= H - 2 && bx < H + TX + 2) ? 1u : 0u) |
                           ((bx >= H && bx < H + TX && by >= L::FY_R0 && by < L::FY_R0 + L::FY_NR) ? 2u : 0u);
       double cm[NDIM];
-      face_eval<NDIM, NDIR, S>(
-          b.a, I.o, c, false, b.a.gamma, cm, fd,
+      bad |= face_eval<NDIM, NDIR, S>(
+          b.a, I.o, c, false, b.a.gamma, cm, fd, true,
           [&](int i, S v) {
             if (i == 0) sm[L::P_OFF + L::P_RT * BW * BH + idx] = v;
             else if (i <= NDIM) sm[L::P_OFF + (L::P_V + i - 1) * BW * BH + idx] = v;
@@ -129,7 +130,14 @@ __device__ __forceinline__ void stage2d_tile(const BatchStageArgs& b, int t, uns
         sm[L::P_OFF + (L::P_B + l) * BW * BH + idx] = ((const S*)b.a.fW[E + 1 + l] + I.o.P)[c];
       }
     }
-    __syncthreads();
+    // a tile takes the divide where its box holds a field, or the instance a c_tot,
+    // out of range (one vote for all its cells)
+    if constexpr (sizeof(S) == 8) {
+      bad = bad || b.a.general || (b.a.visc_on && (ctot_out_of_range(Dy.ctot[0]) || ctot_out_of_range(Dy.ctot[1])));
+      bad = __syncthreads_or(bad);
+    } else {
+      __syncthreads();
+    }
     // ---- phase 2: setnu's face quotients ---------------------------------------
     const double* ctotp = (const double*)Dy.ctot;
     auto pfield = [&](int slot) { return (const S*)(sm + L::P_OFF + slot * BW * BH); };
@@ -152,11 +160,15 @@ __device__ __forceinline__ void stage2d_tile(const BatchStageArgs& b, int t, uns
         // the faces k_nu computes: lo-1 .. hi in every dimension
         if (gx < g.lo[0] - 1 || gx > g.hi[0] || gy < g.lo[1] - 1 || gy > g.hi[1]) continue;
         const int cb = bx + by * BW;
-        const int pos = k == 0 ? gx : gy, lo = g.lo[k], hi = g.hi[k];
+        int fo[6];
+        face_offsets(cb, s, k == 0 ? gx : gy, g.lo[k], g.hi[k], fo);
         S* qo = sm + off + (by - r0) * BW + bx;
+        S md3[L::NQ], md1[L::NQ];
+#pragma unroll
+        for (int j = 0; j < L::NQ; ++j) face_maxima<true>(qsrc(k, j), fo, md3[j], md1[j]);
 #pragma unroll
         for (int j = 0; j < L::NQ; ++j)
-          qo[j * BW * nr] = face_quotient<true>(qsrc(k, j), cb, s, pos, lo, hi, (j == 2 || j == 3) ? p4 : p04);
+          qo[j * BW * nr] = face_ratio((j == 2 || j == 3) ? p4 : p04, md3[j], md1[j]);
       }
     }
     __syncthreads();
@@ -200,7 +212,10 @@ __device__ __forceinline__ void stage2d_tile(const BatchStageArgs& b, int t, uns
         const double qdt = b.stage == 0 ? dt / 2 : b.stage == 1 ? dt / 2 : b.stage == 2 ? dt : dt / 6;
         const double qdt2 = qdt * ((double)(b.a.dmax - b.a.dmin) + 1.0) / (double)g.ndim;
         const double tdep = b.a.driver != DRV_NONE ? sin(omega * tnow) : 0.0;
-        update_cell<NDIM, NDIR, S, 0, true>(b.a, g, I.o, pos, qdt, qdt2, tdep, drvA, numax, &tv);
+        if (sizeof(S) == 8 && bad)
+          update_cell<NDIM, NDIR, S, 0, false, true>(b.a, g, I.o, pos, qdt, qdt2, tdep, drvA, numax, &tv);
+        else
+          update_cell<NDIM, NDIR, S, 0, true, true>(b.a, g, I.o, pos, qdt, qdt2, tdep, drvA, numax, &tv);
       }
     }
     if (b.a.visc_on) block_max_to(&b.dyn[tl.inst].maxnu, numax, shred);

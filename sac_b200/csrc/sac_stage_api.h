@@ -49,7 +49,22 @@ struct Stage2Args {
   const void* F;     // S[ndim*np][N] fluxes, F[d*np+iw]
   const void* R;     // S[NR][N]   setnu face quotients
   const void* X;     // S[n_cross][N] cross-derivative half-sums (single grid), or nullptr
-  const double* dx;  // double[ndim][N]
+  // cell widths with their reciprocals, (dx, 1/dx) pairs of S per dimension: one row
+  // of entries per index along it where the width varies along its own dimension alone
+  // (axis_tab, every Cartesian grid; the rows of width_row), else one per cell [N]
+  const void* xr[3];
+  int axis_tab;
+  // brick flags of the FP64 single grid (k_face): a brick of 8 cells per dimension is
+  // set where a cell within one brick of it holds a field out of range, and its cells
+  // then take the divides; brick strides fst
+  unsigned char* flags;
+  int fst[3];
+  const double* dx[3];  // cell widths per cell (the batch's getdt_courant)
+  unsigned* nbad;       // count of the cells with a field out of range (FP64, 3D)
+  // every cell takes the update's general form: a split sweep (dmin..dmax), a partial
+  // variable list (iwmask), or widths, eta or the step out of range
+  int general;
+  int quiet;            // many cells out of range: the general form's own kernels (FP64, 3D)
   const double* drv; // driver profiles [2][N] or nullptr
   const unsigned long long* ctot;
   unsigned long long* maxnu;
@@ -71,7 +86,6 @@ struct Stage2Args {
   const void* fW[8];      // wct per advanced variable
   const void* fD[6];      // rho+rhob, v.., e173, p'_tot
   const double* fBG[5];   // eb, rhob, bg..
-  const double* fDX[3];   // dx per dimension
   const void* fX[12];     // cross-derivative half-sums per pair
 };
 
@@ -93,7 +107,6 @@ inline void fill_field_ptrs(Stage2Args& a, size_t es) {
   for (int iw = 0; iw < 8; ++iw) a.fW[iw] = (iw < g.np) ? off(a.wct, iw, a.sP) : nullptr;
   for (int i = 0; i < 6; ++i) a.fD[i] = (i < g.ndir + 3) ? off(a.D, i, a.sI) : nullptr;
   for (int i = 0; i < 5; ++i) a.fBG[i] = (i < g.nw - g.np) ? a.bgv + (size_t)i * a.sB : nullptr;
-  for (int d = 0; d < 3; ++d) a.fDX[d] = (d < g.ndim) ? a.dx + (size_t)d * a.sX : nullptr;
   for (int i = 0; i < 12; ++i) a.fX[i] = (i < n_cross(g.ndim)) ? off(a.X, i, a.sI) : nullptr;
 }
 

@@ -8,6 +8,7 @@
 // and square root), so the FP64 instances round exactly as in a batch of their
 // own; the FP32 instances compute with the same rules, which is more exact than
 // the FP32 stage unit's contraction.
+#define SAC_F32_IEEE_DIV 1
 #include "sac_stage.cuh"
 #include "sac_stage2d.cuh"
 
