@@ -161,9 +161,32 @@ __device__ __forceinline__ float tanh_sfu(float x) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// five operations beside the tanh: u = x (c0 + c0 c1 x^2), h = x/2, h + h tanh(u)
 __device__ __forceinline__ float gelu_f(float x) {
-  const float u = 0.7978845608028654f * fmaf(0.044715f * x, x * x, x);
-  return 0.5f * x * (1.0f + tanh_sfu(u));
+  const float u = x * fmaf(0.7978845608028654f * 0.044715f, x * x, 0.7978845608028654f);
+  const float h = 0.5f * x;
+  return fmaf(h, tanh_sfu(u), h);
+}
+// two of them with the packed FP32 operations (the same roundings)
+__device__ __forceinline__ void gelu_2(float& x0, float& x1) {
+  unsigned long long x, q, u, h;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(x0), "f"(x1));
+  asm("mul.rn.f32x2 %0, %1, %1;" : "=l"(q) : "l"(x));
+  const float c1 = 0.7978845608028654f * 0.044715f, c0 = 0.7978845608028654f, hf = 0.5f;
+  unsigned long long k1, k0, kh;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(k1) : "f"(c1));
+  asm("mov.b64 %0, {%1, %1};" : "=l"(k0) : "f"(c0));
+  asm("mov.b64 %0, {%1, %1};" : "=l"(kh) : "f"(hf));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(u) : "l"(k1), "l"(q), "l"(k0));
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(u) : "l"(x), "l"(u));
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(h) : "l"(x), "l"(kh));
+  float u0, u1;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(u0), "=f"(u1) : "l"(u));
+  u0 = tanh_sfu(u0);
+  u1 = tanh_sfu(u1);
+  asm("mov.b64 %0, {%1, %2};" : "=l"(u) : "f"(u0), "f"(u1));
+  asm("fma.rn.f32x2 %0, %1, %2, %1;" : "=l"(h) : "l"(h), "l"(u));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x0), "=f"(x1) : "l"(h));
 }
 __device__ __forceinline__ float gelu_grad_f(float x) {
   const float x2 = x * x;

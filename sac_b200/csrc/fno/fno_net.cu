@@ -30,6 +30,7 @@
 #include "fno_gemm.cuh"
 #include "fno_host.h"
 #include "fno_proj.cuh"
+#include "fno_row.cuh"
 #include "sac_fno.h"
 
 using namespace fno;
@@ -323,22 +324,28 @@ __global__ void __launch_bounds__(256) k_mix_bwd(const float* __restrict__ dpt, 
   }
 }
 
-// out[c] += sum over b, p of d[b][c][p]  (bias gradients)
+// out[c] += sum over b, p of d[b][c][p]  (bias gradients), 8 pixels per load: 32
+// channels of 16 samples of 256 x 256, 129 -> 17 us
 __global__ void __launch_bounds__(256) k_chan_sum(const bf16* __restrict__ d, float* __restrict__ out, int B, int C,
                                                   long P) {
   __shared__ float sh[8];
   const int c = blockIdx.y;
-  float s = 0.f;
-  const long tot = (long)B * P;
-  for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < tot; k += (long)gridDim.x * blockDim.x) {
-    const long b = k / P, p = k % P;
-    s += __bfloat162float(d[(b * C + c) * P + p]);
-  }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  float s[8] = {};
+  const long P8 = P / 8;  // 16-byte loads of 8 pixels: a grid has a multiple of 64
+  for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < P8; q += (long)gridDim.x * blockDim.x)
+#pragma unroll 4
+    for (int b = 0; b < B; ++b) {
+      const uint4 u = __ldg(reinterpret_cast<const uint4*>(d + ((long)b * C + c) * P) + q);
+      const bf16* e = reinterpret_cast<const bf16*>(&u);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) s[k] += __bfloat162float(e[k]);
+    }
+  float t = ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = t;
   __syncthreads();
   if (threadIdx.x == 0) {
-    float t = 0.f;
+    t = 0.f;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += sh[w];
     atomicAdd(out + c, t);
   }
@@ -390,6 +397,46 @@ __global__ void k_mse(const float* __restrict__ y, const bf16* __restrict__ t, b
   if ((threadIdx.x & 31) == 0) atomicAdd(loss, s * inv_n);
 }
 
+// the same with 8 pixels of one channel per thread and one atomic per block (P a
+// multiple of 8, 16-byte aligned y, t and dy): 16 samples of 256 x 256, 67 -> 10 us
+__global__ void __launch_bounds__(256) k_mse8(const float* __restrict__ y, const bf16* __restrict__ t,
+                                              bf16* __restrict__ dy, float* loss, int nbc, int cout, int cpad, int P8,
+                                              float inv_n) {
+  __shared__ float sh[8];
+  float s = 0.f;
+  for (int bc = blockIdx.y; bc < nbc; bc += gridDim.y) {
+    const int c = bc % cpad, b = bc / cpad;
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < P8; q += gridDim.x * blockDim.x) {
+      float g[8] = {};
+      if (c < cout) {
+        const long o = ((long)b * cout + c) * P8 + q;
+        const float4 u0 = reinterpret_cast<const float4*>(y)[2 * o], u1 = reinterpret_cast<const float4*>(y)[2 * o + 1];
+        const uint4 tv = reinterpret_cast<const uint4*>(t)[o];
+        const bf16* te = reinterpret_cast<const bf16*>(&tv);
+        const float v[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float e = v[k] - __bfloat162float(te[k]);
+          s += e * e;
+          g[k] = 2.f * e * inv_n;
+        }
+      }
+      __nv_bfloat162 o2[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) o2[k] = __floats2bfloat162_rn(g[2 * k], g[2 * k + 1]);
+      reinterpret_cast<uint4*>(dy)[(long)bc * P8 + q] = *reinterpret_cast<const uint4*>(o2);
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s = 0.f;
+    for (int w = 0; w < 8; ++w) s += sh[w];
+    atomicAdd(loss, s * inv_n);
+  }
+}
+
 // network input x[b][c][s][f] (bf16, cin channels):
 //   0..nst-1  the state channel times scale[b*nst + c] (normalised perturbation)
 //   nst..     per-sample feature planes feat[b*nfeat + k]
@@ -416,6 +463,70 @@ __global__ void k_features(const T* __restrict__ st, const float* __restrict__ s
     x[k] = __float2bfloat16(v);
   }
 }
+
+// the same with 8 pixels of one channel per thread (P a multiple of 8, 16-byte aligned
+// state and x): 64 samples of 256 x 256, 275 -> 57 us
+template <typename T>
+__global__ void __launch_bounds__(256) k_features8(const T* __restrict__ st, const float* __restrict__ scale,
+                                                   const float* __restrict__ feat, bf16* __restrict__ x, int nbc,
+                                                   int nst, int nfeat, int cin, int S, int F) {
+  const int P8 = (int)((long)S * F / 8), F8 = F / 8;
+  for (int bc = blockIdx.y; bc < nbc; bc += gridDim.y) {
+    const int c = bc % cin, b = bc / cin;
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < P8; q += gridDim.x * blockDim.x) {
+      float v[8];
+      if (c < nst) {
+        const float sc = scale ? scale[b * nst + c] : 1.f;
+        const T* src = st + ((long)b * nst + c) * P8 * 8 + (long)q * 8;
+        if constexpr (sizeof(T) == 4) {
+          const float4 u0 = *reinterpret_cast<const float4*>(src), u1 = *(reinterpret_cast<const float4*>(src) + 1);
+          v[0] = u0.x, v[1] = u0.y, v[2] = u0.z, v[3] = u0.w, v[4] = u1.x, v[5] = u1.y, v[6] = u1.z, v[7] = u1.w;
+        } else {
+          const uint4 u = *reinterpret_cast<const uint4*>(src);
+          const bf16* e = reinterpret_cast<const bf16*>(&u);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) v[k] = __bfloat162float(e[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = v[k] * sc;
+      } else {
+        float u = 0.f;
+        if (c < nst + nfeat) u = feat[b * nfeat + (c - nst)];
+        else if (c == nst + nfeat) u = (float)(q / F8) / (float)S - 0.5f;
+        const bool along_f = c == nst + nfeat + 1;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = along_f ? (float)((q % F8) * 8 + k) / (float)F : u;
+      }
+      __nv_bfloat162 o[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) o[k] = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
+      *reinterpret_cast<uint4*>(x + ((long)bc * P8 + q) * 8) = *reinterpret_cast<const uint4*>(o);
+    }
+  }
+}
+
+// k_apply with 4 pixels per thread (P a multiple of 4, 16-byte aligned state and y):
+// 64 samples of 256 x 256, 73 -> 40 us
+__global__ void __launch_bounds__(256) k_apply4(float* __restrict__ st, const float* __restrict__ y,
+                                                const float* __restrict__ scale, int nbc, int P4) {
+  for (int bc = blockIdx.y; bc < nbc; bc += gridDim.y) {
+    const float sc = scale[bc];
+    float4* d = reinterpret_cast<float4*>(st) + (long)bc * P4;
+    const float4* u = reinterpret_cast<const float4*>(y) + (long)bc * P4;
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < P4; q += gridDim.x * blockDim.x) {
+      const float4 v = u[q];
+      float4 w = d[q];
+      w.x += sc * v.x, w.y += sc * v.y, w.z += sc * v.z, w.w += sc * v.w;
+      d[q] = w;
+    }
+  }
+}
+
+// a grid of rows (y) times chunks (x) for n items of 256 threads each per row
+dim3 grid_rows(long rows, long n) {
+  return dim3((unsigned)std::max<long>(1, std::min<long>((n + 255) / 256, 64)), (unsigned)std::min<long>(rows, 65535));
+}
+bool aligned16p(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
 // st[b][c][p] += scale[b*nst+c] * y[b][c][p]   (apply the predicted increment)
 __global__ void k_apply(float* __restrict__ st, const float* __restrict__ y, const float* __restrict__ scale,
@@ -528,6 +639,91 @@ void c_chanfirst(GemmDesc& d, void* c, int N, long P, int bf) {
   d.c_bf16 = bf;
 }
 
+// one row-kernel launch: persistent, one CTA per SM
+template <int K1, bool SPEC, int ACT, bool NEXT, bool PRE>
+int row_launch(sac_fno* n, const RowArgs& a) {
+  constexpr int smem = RowSmem<K1, SPEC, NEXT>::BYTES;
+  auto* k = k_row<K1, SPEC, ACT, NEXT, PRE>;
+  FK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  int nsm = 148;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, n->cfg.device);
+  const long ntask = (long)a.B * (a.S / 4);
+  k<<<(unsigned)std::min<long>(ntask, nsm), kRowThreads, smem, n->st>>>(a);
+  FK(cudaGetLastError());
+  return 0;
+}
+
+// whether the network's rows fit the row kernel (else: one GEMM per product)
+bool row_ok(const sac_fno* n) { return n->W == kRowN && n->cin == 16 && n->F <= kRowF && n->F % 8 == 0 && n->S % 4 == 0; }
+
+RowArgs row_args(sac_fno* n, int B) {
+  RowArgs a{};
+  a.B = B;
+  a.S = n->S;
+  a.F = n->F;
+  a.err = n->errw;
+  a.wait_tries = n->wait_tries;
+  return a;
+}
+
+// F2 from the row kernel's T[b][s][c][j]: Z[(b,c,j)][r] = sum_s T[b][s][c][j] Fx[r][s]
+int dft_s(sac_fno* n, const bf16* t, float* z, int B) {
+  const int S = n->S, W = n->W;
+  GemmDesc d = gd(kR, W * kJ, S, B);
+  d.a = n->Fx;
+  d.a_m0 = S;
+  d.a_k = 1;
+  d.b = t;
+  d.b_mn_major = 1;
+  d.b_n = 1;
+  d.b_k = (long)W * kJ;
+  d.b_b = (long)S * W * kJ;
+  d.c = z;
+  d.c_m0 = 1;
+  d.c_n = kR;
+  d.c_b = (long)W * kJ * kR;
+  d.err = n->errw;
+  GK(d);
+  return 0;
+}
+
+// spectral mixing of layer l
+int mix_forward(sac_fno* n, int l, int B) {
+  const int W = n->W;
+  if (n->mix_grouped) {
+    const size_t sm = sizeof(float) * kMixQ * (2 * W * W + 2 * B * W);
+    k_mix_fwd<<<n->nmodes / kMixQ, 256, sm, n->st>>>(n->zt[l], n->wb + n->sRr[l].off, n->wb + n->sRi[l].off, n->pt, B,
+                                                     W, n->m2);
+  } else {
+    const size_t sm = sizeof(float) * (2 * W * W + 2 * B * W);
+    k_mix_fwd_mode<<<n->nmodes, 256, sm, n->st>>>(n->zt[l], n->wb + n->sRr[l].off, n->wb + n->sRi[l].off, n->pt, B, W,
+                                                  n->m2);
+  }
+  FK(cudaGetLastError());
+  return 0;
+}
+
+// F4: Y[(b,o)][s][j'] = sum_r P[(b,o),j'][r] Fx[r][s]   (rows (b,o,j'))
+int idft_s(sac_fno* n, const bf16* p, bf16* y, int B) {
+  const int S = n->S, W = n->W;
+  GemmDesc d = gd(B * W * kJ, S, kR);
+  d.a = p;
+  d.a_m0 = kR;
+  d.a_k = 1;
+  d.b = n->Gx;
+  d.b_n = kR;
+  d.b_k = 1;
+  d.c = y;
+  d.c_msplit = kJ;
+  d.c_m0 = 1;
+  d.c_m1 = (long)S * kJ;
+  d.c_n = kJ;
+  d.c_bf16 = 1;
+  d.err = n->errw;
+  GK(d);
+  return 0;
+}
+
 // ---------------------------------------------------------------------------
 // train: keep what the backward pass needs (pre-activations, the input pointer)
 int forward(sac_fno* n, const bf16* x, float* y, int B, bool train) {
@@ -535,6 +731,22 @@ int forward(sac_fno* n, const bf16* x, float* y, int B, bool train) {
   const long P = n->P;
   n->xin = train ? x : nullptr;
   n->Blast = B;
+  // where the shape allows it the lift and the layers' pixel stages run row by row,
+  // with the next layer's DFT along f in the same kernel (fno_row.cuh)
+  const bool rows = row_ok(n) && ((uintptr_t)x & 15) == 0;
+  if (rows) {
+    RowArgs a = row_args(n, B);
+    a.in = x;
+    a.w = n->wb + n->sP.off;
+    a.w_n = n->cin;
+    a.w_k = 1;
+    a.bias = n->w + n->sPb.off;
+    a.out = n->act[0];
+    a.g = n->Fy;
+    a.t = n->tp;
+    int rc = row_launch<16, false, ACT_NONE, true, false>(n, a);
+    if (rc) return rc;
+  } else
   // lift: v0[b][o][p] = sum_c Pw[o][c] x[b][c][p] + pb[o]
   {
     GemmDesc d = gd((int)P, W, n->cin, B);
@@ -549,6 +761,33 @@ int forward(sac_fno* n, const bf16* x, float* y, int B, bool train) {
   }
   for (int l = 0; l < n->L; ++l) {
     const bf16* v = n->act[l];
+    if (rows) {
+      int rc;
+      if ((rc = dft_s(n, n->tp, n->zt[l], B))) return rc;
+      if ((rc = mix_forward(n, l, B))) return rc;
+      if ((rc = idft_s(n, n->pt, n->yb, B))) return rc;
+      RowArgs a = row_args(n, B);
+      a.in = v;
+      a.w = n->wb + n->sW[l].off;
+      a.w_n = W;
+      a.w_k = 1;
+      a.bias = n->w + n->sWb[l].off;
+      a.h = n->Hy;
+      a.y = n->yb;
+      a.out = n->act[l + 1];
+      a.g = n->Fy;
+      a.t = n->tp;
+      if (l == n->L - 1) {
+        rc = row_launch<32, true, ACT_NONE, false, false>(n, a);
+      } else if (train) {
+        a.pre = n->pre[l];
+        rc = row_launch<32, true, ACT_GELU, true, true>(n, a);
+      } else {
+        rc = row_launch<32, true, ACT_GELU, true, false>(n, a);
+      }
+      if (rc) return rc;
+      continue;
+    }
     // F1: T[(b,c)][j][s] = sum_f v[(b,c,s)][f] Fy[j][f]
     {
       GemmDesc d = gd(B * W * S, kJ, F);
@@ -582,37 +821,9 @@ int forward(sac_fno* n, const bf16* x, float* y, int B, bool train) {
       d.err = n->errw;
       GK(d);
     }
-    // spectral mixing
-    {
-      if (n->mix_grouped) {
-        const size_t sm = sizeof(float) * kMixQ * (2 * W * W + 2 * B * W);
-        k_mix_fwd<<<n->nmodes / kMixQ, 256, sm, n->st>>>(n->zt[l], n->wb + n->sRr[l].off, n->wb + n->sRi[l].off,
-                                                         n->pt, B, W, n->m2);
-      } else {
-        const size_t sm = sizeof(float) * (2 * W * W + 2 * B * W);
-        k_mix_fwd_mode<<<n->nmodes, 256, sm, n->st>>>(n->zt[l], n->wb + n->sRr[l].off, n->wb + n->sRi[l].off,
-                                                      n->pt, B, W, n->m2);
-      }
-      FK(cudaGetLastError());
-    }
-    // F4: Y[(b,o)][s][j'] = sum_r P[(b,o),j'][r] Fx[r][s]   (rows (b,o,j'))
-    {
-      GemmDesc d = gd(B * W * kJ, S, kR);
-      d.a = n->pt;
-      d.a_m0 = kR;
-      d.a_k = 1;
-      d.b = n->Gx;
-      d.b_n = kR;
-      d.b_k = 1;
-      d.c = n->yb;
-      d.c_msplit = kJ;
-      d.c_m0 = 1;
-      d.c_m1 = (long)S * kJ;
-      d.c_n = kJ;
-      d.c_bf16 = 1;
-      d.err = n->errw;
-      GK(d);
-    }
+    int rc;
+    if ((rc = mix_forward(n, l, B))) return rc;
+    if ((rc = idft_s(n, n->pt, n->yb, B))) return rc;
     // F5 and F6 in one GEMM where a 128-row tile of pixels lies in one row s (F a
     // multiple of 128): z[b][o][p] = sum_i W[o][i] v[b][i][p] + sum_j' Hy[f][j'] Y[(b,o),s][j']
     // + b[o] accumulates both products in the tile's TMEM accumulator, so the
@@ -773,7 +984,7 @@ int wgrad(sac_fno* n, const bf16* dout, int R, const bf16* in, int C, float* gou
 }
 
 int bias_grad(sac_fno* n, const bf16* d, int C, float* out, int B) {
-  dim3 grid(64, C);
+  const dim3 grid((unsigned)std::min<long>(64, (n->P / 8 + 255) / 256), C);
   k_chan_sum<<<grid, 256, 0, n->st>>>(d, out, B, C, n->P);
   FK(cudaGetLastError());
   return 0;
@@ -1258,7 +1469,12 @@ int sac_fno_backward(sac_fno* n, const void* dy) {
 int sac_fno_mse(sac_fno* n, const float* y, const void* target, void* dy, float* loss, int B) {
   if (!n || !y || !target || !dy || !loss) return fail(n, "sac_fno_mse: null argument");
   const long tot = (long)B * n->cout * n->P;
-  k_mse<<<grid_for((long)B * n->cpad * n->P), 256, 0, n->st>>>(y, (const bf16*)target, (bf16*)dy, loss, B,
+  if (aligned16p(y) && aligned16p(target) && aligned16p(dy))
+    k_mse8<<<grid_rows((long)B * n->cpad, n->P / 8), 256, 0, n->st>>>(y, (const bf16*)target, (bf16*)dy, loss,
+                                                                     B * n->cpad, n->cout, n->cpad, (int)(n->P / 8),
+                                                                     1.0f / (float)tot);
+  else
+    k_mse<<<grid_for((long)B * n->cpad * n->P), 256, 0, n->st>>>(y, (const bf16*)target, (bf16*)dy, loss, B,
                                                                n->cout, n->cpad, n->P, 1.0f / (float)tot);
   FK(cudaGetLastError());
   return 0;
@@ -1293,7 +1509,15 @@ int sac_fno_features(sac_fno* n, const void* state, int state_bf16, const float*
   if (!n || !state || !x) return fail(n, "sac_fno_features: null argument");
   if (nst + nfeat + 2 > n->cin) return fail(n, "sac_fno_features: too many channels for cin");
   const long tot = (long)B * n->cin * n->P;
-  if (state_bf16)
+  if (aligned16p(state) && aligned16p(x)) {  // whole 16-byte chunks (the planes are multiples of 64 pixels)
+    const dim3 grid = grid_rows((long)B * n->cin, n->P / 8);
+    if (state_bf16)
+      k_features8<bf16><<<grid, 256, 0, n->st>>>((const bf16*)state, scale, feat, (bf16*)x, B * n->cin, nst, nfeat,
+                                                 n->cin, n->S, n->F);
+    else
+      k_features8<float><<<grid, 256, 0, n->st>>>((const float*)state, scale, feat, (bf16*)x, B * n->cin, nst, nfeat,
+                                                  n->cin, n->S, n->F);
+  } else if (state_bf16)
     k_features<bf16><<<grid_for(tot), 256, 0, n->st>>>((const bf16*)state, scale, feat, (bf16*)x, B, nst, nfeat,
                                                        n->cin, n->S, n->F);
   else
@@ -1305,7 +1529,10 @@ int sac_fno_features(sac_fno* n, const void* state, int state_bf16, const float*
 
 int sac_fno_apply(sac_fno* n, float* state, const float* y, const float* scale, int B, int nst) {
   if (!n || !state || !y || !scale) return fail(n, "sac_fno_apply: null argument");
-  k_apply<<<grid_for((long)B * nst * n->P), 256, 0, n->st>>>(state, y, scale, B, nst, n->P);
+  if (aligned16p(state) && aligned16p(y))
+    k_apply4<<<grid_rows((long)B * nst, n->P / 4), 256, 0, n->st>>>(state, y, scale, B * nst, (int)(n->P / 4));
+  else
+    k_apply<<<grid_for((long)B * nst * n->P), 256, 0, n->st>>>(state, y, scale, B, nst, n->P);
   FK(cudaGetLastError());
   return 0;
 }

@@ -124,8 +124,9 @@ __global__ void __launch_bounds__(kThreads, 3) k_proj_infer(const ProjArgs a) {
       uint32_t h[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const float x0 = gelu_f(__uint_as_float(v[2 * j]) + b1s[cc + 2 * j]);
-        const float x1 = gelu_f(__uint_as_float(v[2 * j + 1]) + b1s[cc + 2 * j + 1]);
+        float x0 = __uint_as_float(v[2 * j]) + b1s[cc + 2 * j];
+        float x1 = __uint_as_float(v[2 * j + 1]) + b1s[cc + 2 * j + 1];
+        gelu_2(x0, x1);
         const __nv_bfloat162 pr = __floats2bfloat162_rn(x0, x1);
         h[j] = *reinterpret_cast<const uint32_t*>(&pr);
       }

@@ -1,0 +1,74 @@
+"""The FNO's row kernel and its vectorised streaming kernels at the edges of their ranges.
+
+Forward passes against the float64 oracle on grids with one and two pixel tiles per
+row, ragged rows, few and many rows per CTA, and just past the row kernel's width (one
+GEMM per product); the bound is the one of the BF16 network (2e-2 relative L2)."""
+import numpy as np
+import pytest
+
+from oracle import fno_ref
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def _net(S, F, B):
+    from sac_b200 import fno_abi
+
+    return fno_abi.Net(S=S, F=F, max_batch=B, seed=3)
+
+
+@pytest.mark.parametrize("S,F,B", [(56, 56, 1), (56, 128, 1), (64, 136, 3), (200, 120, 5), (104, 248, 2), (64, 256, 1),
+                                   (56, 264, 1)])
+def test_forward_matches_the_oracle(S, F, B):
+    net, lay = _net(S, F, B), fno_ref.Layout(32, 4, 16, 6, 128)
+    x = torch.randn(B, 16, S, F, generator=torch.Generator().manual_seed(9)).to(torch.bfloat16)
+    xd, y = x.cuda(), torch.full((B, 6, S, F), float("nan"), device="cuda")
+    y2 = y.clone()
+    torch.cuda.synchronize()
+    net.forward(xd.data_ptr(), y.data_ptr(), B)
+    net.infer(xd.data_ptr(), y2.data_ptr(), B)
+    net.check()
+    theta = net.get_params().astype(np.float64)
+    # the network reads BF16 weights (biases stay FP32)
+    for name, (o, n) in lay.segs.items():
+        if not name.endswith("b") and not (name[-1].isdigit() and name.startswith("Wb")):
+            theta[o:o + n] = fno_ref.bf16_round(theta[o:o + n])
+    want, _ = fno_ref.forward(lay, theta, x.double().numpy())
+    got = y.cpu().double().numpy()
+    assert np.linalg.norm(got - want) / np.linalg.norm(want) < 2e-2
+    assert torch.equal(y, y2)
+
+
+def test_unaligned_buffers_give_the_same():
+    """features, apply and mse with buffers off the 16-byte boundary take the scalar
+    kernels: the same values (the loss up to the order of its sum)."""
+    S, F, B = 56, 72, 2
+    net = _net(S, F, B)
+    g = torch.Generator("cuda").manual_seed(4)
+
+    def buf(shape, dtype, off):
+        n = int(np.prod(shape))
+        return torch.zeros(n + off, dtype=dtype, device="cuda")[off:].view(shape)
+
+    st = torch.randn(B, 6, S, F, generator=g, device="cuda")
+    sc, feat = torch.rand(B * 6, generator=g, device="cuda"), torch.rand(B * 4, generator=g, device="cuda")
+    y, t = torch.randn(B, 6, S, F, generator=g, device="cuda"), torch.randn(B, 6, S, F, generator=g, device="cuda")
+    out = []
+    for off in (0, 1):
+        s, yy = buf(st.shape, torch.float32, off), buf(y.shape, torch.float32, off)
+        tt = buf(t.shape, torch.bfloat16, off)
+        x, dy = buf((B, 16, S, F), torch.bfloat16, off), buf((B, 8, S, F), torch.bfloat16, off)
+        s.copy_(st), yy.copy_(y), tt.copy_(t)
+        loss = torch.zeros(1, device="cuda")
+        torch.cuda.synchronize()
+        net.features(s.data_ptr(), False, sc.data_ptr(), feat.data_ptr(), 4, x.data_ptr(), B, 6)
+        net.apply(s.data_ptr(), yy.data_ptr(), sc.data_ptr(), B, 6)
+        net.mse(yy.data_ptr(), tt.data_ptr(), dy.data_ptr(), loss.data_ptr(), B)
+        net.check()
+        torch.cuda.synchronize()
+        out.append((x.clone(), s.clone(), dy.clone(), float(loss)))
+    for a, b in zip(out[0][:3], out[1][:3]):
+        assert torch.equal(a, b)
+    # FP32 sums of 48384 squares in another order: n^0.5 * 2^-24 relative, with room
+    assert abs(out[0][3] - out[1][3]) <= 1e-4 * abs(out[1][3])
