@@ -67,9 +67,10 @@ struct sac_ctx {
   // 0 maxnu, 1 courant, 2..4 ctot, 5 cells out of range of the last step (32 bits); then
   // the FP64 stage's brick flags (one memset clears ctot and the flags)
   unsigned long long* red = nullptr;
-  // that count on the host (pinned; FP64 3D) as of a recent step: it chooses between
-  // kernels with the same results, so its age does not matter
-  unsigned* h_nbad = nullptr;
+  // pinned words: maxnu and courant as getdt copied them, and the count above (FP64 3D)
+  // as of a recent step; the count chooses between kernels with the same results, so
+  // its age does not matter
+  unsigned long long* h_red = nullptr;
   size_t nflags = 0;  // bytes of flags (0: FP32)
   unsigned long long* kp = nullptr;   // keeppositive's words (smallfix only), see k_keeppos_scan
   int it_now = 0;                     // the step number last passed to sac_getdt or sac_advect
@@ -196,6 +197,8 @@ bool visc_on(const sac_ctx* c) {
   if (c->par.user == SAC_USR_NONE) return false;
   return std::fabs(c->par.nu) > smalldouble;
 }
+// the FP64 3D stage counts its cells out of range
+bool count_bad(const sac_ctx* c) { return c->g.ndim == 3 && c->prec == SAC_PREC_FP64; }
 bool grav_module(int u) {
   return u == SAC_USR_SLOG || u == SAC_USR_GRAVVISC || u == SAC_USR_STRAT || u == SAC_USR_TUBE;
 }
@@ -210,8 +213,8 @@ void release(sac_ctx* c) {
   c->BG = c->x = c->dx = c->drv = c->stg = c->fixB = nullptr;
   c->D = c->F = c->R = c->X = c->xr = nullptr;
   c->red = c->kp = nullptr;
-  if (c->h_nbad) cudaFreeHost(c->h_nbad);
-  c->h_nbad = nullptr;
+  if (c->h_red) cudaFreeHost(c->h_red);
+  c->h_red = nullptr;
   c->d_type = nullptr;
   c->d_fixed = nullptr;
 }
@@ -316,12 +319,100 @@ void launch_bound(sac_ctx* c, const BcArgs& b, int nvar) {
   ghost_slabs(g, ns);
   const long tot = ns[0] + ns[1] + ns[2];
   if (tot == 0) return;
-  const int bs = 256;
   Prof pr(c, SAC_K_BOUND);
-  k_bound<S><<<(unsigned)((tot + bs - 1) / bs), bs, 0, c->stream>>>(b, ns[0], ns[1], ns[2], nvar);
+  // a thread per cell and variable: one thread's variables are resolved one after
+  // another, each a chain of dependent loads (15 -> 5 us at 251x187, 47 -> 39 at 128^3)
+  k_bound<S><<<dim3((unsigned)((tot + 63) / 64), nvar), 64, 0, c->stream>>>(b, ns[0], ns[1], ns[2]);
 }
 
 sac_status keeppositive(sac_ctx* c, void* A);
+
+// the arguments of one stage: out = base + qdt R(wct) (flux: cd4, with the fluxes of
+// the dimensions dmin..dmax; otherwise the sources alone)
+template <typename S>
+Stage2Args stage_args(sac_ctx* c, bool flux, double qdt, int dmin, int dmax, double qt, const void* wct,
+                      const void* base, void* out, unsigned mask, int epi, void* aux1, const void* aux2) {
+  const Geom& g = c->g;
+  const int u = c->par.user;
+  const bool visc = c->par.sourceunsplit && visc_on(c);
+  Stage2Args a{};
+  a.g = g;
+  a.wct = wct;
+  a.bgv = c->BG;
+  a.base = base;
+  a.out = out;
+  a.aux1 = aux1;
+  a.aux2 = aux2;
+  a.D = c->D;
+  a.F = c->F;
+  a.R = c->R;
+  a.X = c->X;
+  const size_t pair = 2 * c->es;
+  for (int d = 0; d < g.ndim; ++d) a.xr[d] = (const char*)c->xr + pair * c->xr_off[d];
+  a.axis_tab = c->axis_tab;
+  a.flags = (unsigned char*)(c->red + 6);
+  a.fst[0] = 1;
+  a.fst[1] = (g.n[0] + 7) / 8;
+  a.fst[2] = a.fst[1] * ((g.n[1] + 7) / 8);
+  a.drv = c->drv;
+  a.ctot = c->red + 2;
+  a.maxnu = c->red;
+  a.qdt = qdt;
+  // sources inside centdiff4 carry qdt*(idimmax-idimmin+1)/ndim, src/vaccd.t:73-75;
+  // advect1 'source' passes qdt unchanged
+  a.qdt2 = flux ? qdt * ((double)(dmax - dmin) + 1.0) / (double)g.ndim : qdt;
+  a.gamma = c->par.gamma;
+  for (int d = 0; d < 3; ++d) a.grav[d] = (d < g.ndim) ? c->par.grav[d] : 0.0;
+  if (c->par.alias_nu_grav3 && g.ndim == 3) a.grav[2] = 1.0;
+  a.dmin = flux ? dmin : 1;
+  a.dmax = flux ? dmax : 0;
+  a.iwmask = mask;
+  a.general = a.dmin != 0 || a.dmax != g.ndim - 1 || mask != (1u << g.np) - 1u || !c->widths_ok;
+  for (int d = 0; d < 3; ++d)
+    for (int s2 = 0; s2 < 2; ++s2) a.zero1[d][s2] = c->zero1[d][s2];
+  a.grav_on = (c->par.sourceunsplit && grav_module(u)) ? 1 : 0;
+  a.visc_on = visc ? 1 : 0;
+  // addsource (src/vacphys.mhd0.t:225-258): resistivity when |eta| > smalldouble,
+  // Powell's term when divbfix is set, compiled out of 1D builds ({^NOONED}, :255)
+  a.res_on = (c->par.sourceunsplit && std::fabs(c->par.eta) > smalldouble) ? 1 : 0;
+  a.res_compact = c->par.compactres ? 1 : 0;
+  a.eta = c->par.eta;
+  a.divb_on = (c->par.sourceunsplit && c->par.divbfix && g.ndim > 1) ? 1 : 0;
+  // the resistive terms divide products with eta and the step
+  if (a.res_on && (!(a.eta >= 0x1p-60 && a.eta <= 0x1p60) ||
+                   !(std::fabs(a.qdt2) >= 0x1p-80 && std::fabs(a.qdt2) <= 0x1p60)))
+    a.general = 1;
+  a.nbad = (unsigned*)(c->red + 5);
+  a.quiet = count_bad(c) && (long)*(volatile unsigned*)(c->h_red + 2) > g.ncell / kQuietShare ? 1 : 0;
+  a.driver = DRV_NONE;
+  if (c->par.sourceunsplit && c->drv) {
+    if (u == SAC_USR_SLOG && g.ndim == 3) {
+      a.driver = DRV_SLOG;  // tdep=SIN(qt*2*pi/s_period), src/vacusr.f:1321
+      a.tdep = std::sin(qt * 2.0 * (double)3.1415926535897932384626433832795f / 240.0);
+    } else if (u == SAC_USR_STRAT || u == SAC_USR_TUBE) {
+      a.driver = (u == SAC_USR_STRAT) ? DRV_STRAT : DRV_TUBE;
+      a.tdep = std::sin(c->par.userpar[1] * qt);
+    }
+    a.drvA = c->drvA;
+  }
+  a.epi = epi;
+  return a;
+}
+
+// the boundary fill of a stage's output, with the RK4 combinations fused into it
+BcArgs stage_bc(sac_ctx* c, const void* base, void* out, int epi, void* aux1, const void* aux2) {
+  BcArgs b = bc_args(c, out);
+  if (epi == EPI_RK4_S3) {
+    b.mode = 1;
+    b.aux1 = aux1;
+    b.aux2 = aux2;
+    b.basep = base;
+  } else if (epi == EPI_RK4_S4) {
+    b.mode = 2;
+    b.aux1 = aux1;
+  }
+  return b;
+}
 
 // advect1 (src/vac.t:490-549): out = base + qdt R(wct), then getboundary(out)
 template <typename S>
@@ -330,71 +421,10 @@ sac_status advect1_t(sac_ctx* c, const std::string& method, double qdt, int dmin
                      const void* aux2) {
   const Geom& g = c->g;
   if (method == "cd4" || method == "source") {
-    const bool flux = (method == "cd4");
-    const int u = c->par.user;
-    const bool visc = c->par.sourceunsplit && visc_on(c);
     CK(cudaMemsetAsync(c->red + 2, 0, 4 * sizeof(unsigned long long) + c->nflags, c->stream));
-    Stage2Args a{};
-    a.g = g;
-    a.wct = wct;
-    a.bgv = c->BG;
-    a.base = base;
-    a.out = out;
-    a.aux1 = aux1;
-    a.aux2 = aux2;
-    a.D = c->D;
-    a.F = c->F;
-    a.R = c->R;
-    a.X = c->X;
-    const size_t pair = 2 * c->es;
-    for (int d = 0; d < g.ndim; ++d) a.xr[d] = (const char*)c->xr + pair * c->xr_off[d];
-    a.axis_tab = c->axis_tab;
-    a.flags = (unsigned char*)(c->red + 6);
-    a.fst[0] = 1;
-    a.fst[1] = (g.n[0] + 7) / 8;
-    a.fst[2] = a.fst[1] * ((g.n[1] + 7) / 8);
-    a.drv = c->drv;
-    a.ctot = c->red + 2;
-    a.maxnu = c->red;
-    a.qdt = qdt;
-    // sources inside centdiff4 carry qdt*(idimmax-idimmin+1)/ndim, src/vaccd.t:73-75;
-    // advect1 'source' passes qdt unchanged
-    a.qdt2 = flux ? qdt * ((double)(dmax - dmin) + 1.0) / (double)g.ndim : qdt;
-    a.gamma = c->par.gamma;
-    for (int d = 0; d < 3; ++d) a.grav[d] = (d < g.ndim) ? c->par.grav[d] : 0.0;
-    if (c->par.alias_nu_grav3 && g.ndim == 3) a.grav[2] = 1.0;
-    a.dmin = flux ? dmin : 1;
-    a.dmax = flux ? dmax : 0;
-    a.iwmask = mask;
-    a.general = a.dmin != 0 || a.dmax != g.ndim - 1 || mask != (1u << g.np) - 1u || !c->widths_ok;
-    for (int d = 0; d < 3; ++d)
-      for (int s2 = 0; s2 < 2; ++s2) a.zero1[d][s2] = c->zero1[d][s2];
-    a.grav_on = (c->par.sourceunsplit && grav_module(u)) ? 1 : 0;
-    a.visc_on = visc ? 1 : 0;
-    // addsource (src/vacphys.mhd0.t:225-258): resistivity when |eta| > smalldouble,
-    // Powell's term when divbfix is set, compiled out of 1D builds ({^NOONED}, :255)
-    a.res_on = (c->par.sourceunsplit && std::fabs(c->par.eta) > smalldouble) ? 1 : 0;
-    a.res_compact = c->par.compactres ? 1 : 0;
-    a.eta = c->par.eta;
-    a.divb_on = (c->par.sourceunsplit && c->par.divbfix && g.ndim > 1) ? 1 : 0;
-    // the resistive terms divide products with eta and the step
-    if (a.res_on && (!(a.eta >= 0x1p-60 && a.eta <= 0x1p60) ||
-                     !(std::fabs(a.qdt2) >= 0x1p-80 && std::fabs(a.qdt2) <= 0x1p60)))
-      a.general = 1;
-    a.nbad = (unsigned*)(c->red + 5);
-    a.quiet = c->h_nbad && (long)*(volatile unsigned*)c->h_nbad > g.ncell / kQuietShare ? 1 : 0;
-    a.driver = DRV_NONE;
-    if (c->par.sourceunsplit && c->drv) {
-      if (u == SAC_USR_SLOG && g.ndim == 3) {
-        a.driver = DRV_SLOG;  // tdep=SIN(qt*2*pi/s_period), src/vacusr.f:1321
-        a.tdep = std::sin(qt * 2.0 * (double)3.1415926535897932384626433832795f / 240.0);
-      } else if (u == SAC_USR_STRAT || u == SAC_USR_TUBE) {
-        a.driver = (u == SAC_USR_STRAT) ? DRV_STRAT : DRV_TUBE;
-        a.tdep = std::sin(c->par.userpar[1] * qt);
-      }
-      a.drvA = c->drvA;
-    }
-    a.epi = epi;
+    const Stage2Args a =
+        stage_args<S>(c, method == "cd4", qdt, dmin, dmax, qt, wct, base, out, mask, epi, aux1, aux2);
+    const bool visc = a.visc_on != 0;
     {
       Prof pr(c, SAC_K_PREP);
       launch_face<S>(a, visc ? 1 : 0, c->stream);
@@ -417,18 +447,37 @@ sac_status advect1_t(sac_ctx* c, const std::string& method, double qdt, int dmin
     sac_status st = keeppositive(c, out);
     if (st != SAC_OK) return st;
   }
-  BcArgs b = bc_args(c, out);
-  if (epi == EPI_RK4_S3) {
-    b.mode = 1;
-    b.aux1 = aux1;
-    b.aux2 = aux2;
-    b.basep = base;
-  } else if (epi == EPI_RK4_S4) {
-    b.mode = 2;
-    b.aux1 = aux1;
-  }
+  const BcArgs b = stage_bc(c, base, out, epi, aux1, aux2);
   launch_bound<S>(c, b, g.np);
   CK(cudaGetLastError());
+  return SAC_OK;
+}
+
+// Whether a 'fourstep' step runs as one launch (k_step1d): a 1D grid of 64 cells (below,
+// a CTA's segment would not hold setnu's mirrored cells) to what fits in the cluster's
+// shared memory (about 17000 in FP64), the default sources, an unsplit sweep over all
+// variables
+bool step1d_ok(const sac_ctx* c, const std::string& m, unsigned mask) {
+  const Geom& g = c->g;
+  return g.ndim == 1 && m == "cd4" && mask == (1u << g.np) - 1u && !c->regions && !c->par.smallfix &&
+         !(c->par.sourceunsplit && std::fabs(c->par.eta) > smalldouble) && g.n[0] >= 64 && g.n[0] < 30000 &&
+         step1d_smem(g.np, g.n[0], c->es) <= kStep1dSmem;
+}
+
+template <typename S>
+sac_status step1d(sac_ctx* c, double dt, double t, unsigned mask) {
+  void *w = c->P[0], *w1 = c->P[1], *w2 = c->P[2], *w3 = c->P[3];
+  const void* wct[4] = {w, w1, w2, w3};
+  void* out[4] = {w1, w2, w3, w};
+  const double qdt[4] = {dt / 2, dt / 2, dt, dt / 6};
+  const int epi[4] = {EPI_PLAIN, EPI_PLAIN, EPI_RK4_S3, EPI_RK4_S4};
+  Step1dArgs p{};
+  for (int s = 0; s < 4; ++s) {
+    p.st[s] = stage_args<S>(c, true, qdt[s], 0, 0, t, wct[s], w, out[s], mask, epi[s], w1, w2);
+    p.bc[s] = stage_bc(c, w, out[s], epi[s], w1, w2);
+  }
+  Prof pr(c, SAC_K_STAGE);
+  CK(launch_step1d<S>(p, c->stream));
   return SAC_OK;
 }
 
@@ -943,10 +992,8 @@ sac_status sac_set_grid(sac_ctx* c, int ndim, int ndir, const int ixGhi[3], cons
   }
   CK(cudaMalloc(&c->red, 6 * sizeof(unsigned long long) + c->nflags));
   CK(cudaMemsetAsync(c->red, 0, 6 * sizeof(unsigned long long) + c->nflags, c->stream));
-  if (ndim == 3 && c->prec == SAC_PREC_FP64) {
-    CK(cudaMallocHost(&c->h_nbad, sizeof(unsigned)));
-    *c->h_nbad = 0;
-  }
+  CK(cudaMallocHost(&c->h_red, 3 * sizeof(unsigned long long)));
+  std::memset(c->h_red, 0, 3 * sizeof(unsigned long long));
   if (c->par.smallfix) {
     static const unsigned long long kp0[5] = {0, ~0ull, 0, 0, ~0ull};
     CK(cudaMalloc(&c->kp, sizeof(kp0)));
@@ -1236,6 +1283,7 @@ static sac_status getdt_impl(sac_ctx* c, double* dt, int it, bool static_scratch
   }
   c->it_now = it;
   const Geom& g = c->g;
+  bool have_maxnu = false;
   double d;
   if (c->par.dtpar > 0.0) {
     d = c->par.dtpar;
@@ -1249,7 +1297,6 @@ static sac_status getdt_impl(sac_ctx* c, double* dt, int it, bool static_scratch
         return fail(c, SAC_ERR_NONFINITE, "non-finite wave speed in getdt_courant");
       if (courantmax > smalldouble) d = std::min(d, c->par.courantpar / courantmax);
     } else if (c->par.courantpar > 0.0) {  // getdt_courant, src/vac.t:641-699
-      CK(cudaMemsetAsync(c->red + 1, 0, sizeof(unsigned long long), c->stream));
       const long nm = (long)(g.hi[0] - g.lo[0] + 1) * (g.hi[1] - g.lo[1] + 1) * (g.hi[2] - g.lo[2] + 1);
       const int bs = 256;
       const unsigned nb = (unsigned)std::min<long>((nm + bs - 1) / bs, 148L * 16);
@@ -1269,11 +1316,13 @@ static sac_status getdt_impl(sac_ctx* c, double* dt, int it, bool static_scratch
       else
         launch(0.0);
       }
-      unsigned long long bits = 0;
-      CK(cudaMemcpyAsync(&bits, c->red + 1, sizeof(bits), cudaMemcpyDeviceToHost, c->stream));
+      // both maxima in one copy and one wait; courant starts the next call at zero
+      CK(cudaMemcpyAsync(c->h_red, c->red, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
+      CK(cudaMemsetAsync(c->red + 1, 0, sizeof(unsigned long long), c->stream));
       CK(cudaStreamSynchronize(c->stream));
+      have_maxnu = true;
       double courantmax;
-      std::memcpy(&courantmax, &bits, sizeof(double));
+      std::memcpy(&courantmax, c->h_red + 1, sizeof(double));
       if (!(courantmax == courantmax) || std::isinf(courantmax))
         return fail(c, SAC_ERR_NONFINITE, "non-finite wave speed in getdt_courant");
       if (courantmax > smalldouble) d = std::min(d, c->par.courantpar / courantmax);
@@ -1285,11 +1334,12 @@ static sac_status getdt_impl(sac_ctx* c, double* dt, int it, bool static_scratch
     const int u = c->par.user;
     if (grav_module(u)) {  // getdt_special of the Slog/gravity user files
       if (visc_on(c)) {    // getdt_visc, src/vacusr.viscosity.t:509-542
-        unsigned long long bits = 0;
-        CK(cudaMemcpyAsync(&bits, c->red, sizeof(bits), cudaMemcpyDeviceToHost, c->stream));
-        CK(cudaStreamSynchronize(c->stream));
+        if (!have_maxnu) {
+          CK(cudaMemcpyAsync(c->h_red, c->red, sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
+          CK(cudaStreamSynchronize(c->stream));
+        }
         double maxviscoef;
-        std::memcpy(&maxviscoef, &bits, sizeof(double));
+        std::memcpy(&maxviscoef, c->h_red, sizeof(double));
         if (!(maxviscoef == maxviscoef)) return fail(c, SAC_ERR_NONFINITE, "non-finite hyperdiffusion coefficient");
         c->par.dtdiffpar = 0.25;
         for (int dd = 0; dd < g.ndim; ++dd) {
@@ -1377,6 +1427,11 @@ sac_status sac_advect(sac_ctx* c, const char* method, const int* iws, int idimmi
       else
         k_rk4_final<double><<<592, 256, 0, c->stream>>>((double*)w, (const double*)w1, n);
     }
+  } else if (ta == "fourstep" && step1d_ok(c, m, mask)) {
+    if (c->prec == SAC_PREC_FP32)
+      RUN(step1d<float>(c, dt, t, mask));
+    else
+      RUN(step1d<double>(c, dt, t, mask));
   } else if (ta == "fourstep") {
     RUN(advect1(c, m, dt / 2, dmin, dmax, t, w, w, w1, mask));
     RUN(advect1(c, m, dt / 2, dmin, dmax, t, w1, w, w2, mask));
@@ -1431,8 +1486,8 @@ sac_status sac_advect(sac_ctx* c, const char* method, const int* iws, int idimmi
     return fail(c, SAC_ERR_UNSUPPORTED, "typeadvance=" + ta);
   }
 #undef RUN
-  if (c->h_nbad)
-    CK(cudaMemcpyAsync(c->h_nbad, c->red + 5, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+  if (count_bad(c))
+    CK(cudaMemcpyAsync(c->h_red + 2, c->red + 5, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaGetLastError());
   return SAC_OK;
 }

@@ -459,11 +459,11 @@ __device__ void bound_cell(const BcArgs& a, long t, const long ns[3], int iw0, i
 // __grid_constant__: the resolver takes the parameters by reference, which
 // would otherwise copy the whole struct to each thread's stack
 template <typename S>
-__global__ void k_bound(const __grid_constant__ BcArgs a, long nslab0, long nslab1, long nslab2, int nvar) {
+__global__ void k_bound(const __grid_constant__ BcArgs a, long nslab0, long nslab1, long nslab2) {
   const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
   const long ns[3] = {nslab0, nslab1, nslab2};
   if (t >= nslab0 + nslab1 + nslab2) return;
-  bound_cell<S>(a, t, ns, 0, nvar);
+  bound_cell<S>(a, t, ns, blockIdx.y, blockIdx.y + 1);  // one variable per block row
 }
 
 // batched: persistent CTAs of 256 threads walk the ghost chunks of all instances.

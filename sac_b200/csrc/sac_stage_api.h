@@ -128,6 +128,24 @@ void launch_update(const Stage2Args& a, cudaStream_t st);
 template <typename S>
 void launch_cross(const Stage2Args& a, cudaStream_t st);
 
+// a whole RK4 step of a small 1D grid in one launch (sac_step1d.cuh): the four stages'
+// arguments and boundary fills; the largest shared memory such a grid may take
+struct Step1dArgs {
+  Stage2Args st[4];
+  BcArgs bc[4];
+};
+constexpr int kStep1dCtas = 8, kStep1dSmem = 220 * 1024;
+// the cells of one CTA; its shared memory: the stencil fields of np advanced variables
+// and a byte for each cell of the segment and three to either side
+__host__ __device__ inline int step1d_segment(int n) { return (n + kStep1dCtas - 1) / kStep1dCtas; }
+inline int step1d_smem(int np, int n, size_t es) {
+  return (5 + (np - 1) + 3) * (step1d_segment(n) + 6) * (int)es + step1d_segment(n) + 6;
+}
+template <typename S>
+cudaError_t launch_step1d(const Step1dArgs& p, cudaStream_t st);
+extern template cudaError_t launch_step1d<double>(const Step1dArgs&, cudaStream_t);
+extern template cudaError_t launch_step1d<float>(const Step1dArgs&, cudaStream_t);
+
 template <typename S>
 void launch_batch_face(const BatchStageArgs& b, double gamma, cudaStream_t st);
 template <typename S>

@@ -2,6 +2,7 @@
 // built with contraction and approximate single-precision division.
 #include "sac_stage.cuh"
 #include "sac_stage2d.cuh"
+#include "sac_step1d.cuh"
 
 namespace sacgpu {
 template void launch_face<float>(const Stage2Args&, int, cudaStream_t);
@@ -14,4 +15,5 @@ template void launch_batch_update<float>(const BatchStageArgs&, dim3, cudaStream
 template void launch_batch_courant<float>(const BatchStageArgs&, double, cudaStream_t);
 template void launch_batch_ctot<float>(const BatchStageArgs&, cudaStream_t);
 template cudaError_t launch_batch_stage2d<float>(const BatchStageArgs&, int, cudaStream_t);
+template cudaError_t launch_step1d<float>(const Step1dArgs&, cudaStream_t);
 }  // namespace sacgpu
