@@ -68,8 +68,9 @@ __device__ __forceinline__ void width_at(const Stage2Args& a, const Offs& o, int
 //
 // Every quotient has the total density as its divisor: one reciprocal and the
 // three-operation form (qdiv) instead of about 30 divides per cell.  A cell with a
-// field out of range takes the divide, and is reported (FP64 storage; FP32 values
-// squared or cubed stay inside the range of FP64).  Measured with the update's form
+// field out of range takes the divide, and is reported (FP64 storage; finite FP32
+// values squared or cubed stay inside the range of FP64, so there only a density
+// without a reciprocal and non-finite fields take it).  Measured with the update's form
 // of the same (launch_update).
 template <int NDIM, int NDIR, typename S, class DOut, class FOut>
 __device__ __forceinline__ bool face_eval(const Stage2Args& a, const Offs& o, long c, bool mesh, double gamma,
@@ -94,6 +95,12 @@ __device__ __forceinline__ bool face_eval(const Stage2Args& a, const Offs& o, lo
     bad = !(fabs(rt) >= 0x1p-100 && fabs(rt) < 0x1p100) || out_of_range(rho) || out_of_range(e) || out_of_range(eb) || out_of_range(rhob);
 #pragma unroll
     for (int C = 0; C < NDIR; ++C) bad = bad || out_of_range(m[C]) || out_of_range(b[C]) || out_of_range(bg[C]);
+  }
+  if constexpr (sizeof(S) == 4) {  // a zero or huge density, an Inf or NaN: the quotient's own Inf or NaN
+    float sum = (float)rho + (float)e + (float)eb;
+#pragma unroll
+    for (int C = 0; C < NDIR; ++C) sum += (float)m[C] + (float)b[C] + (float)bg[C];
+    bad = !(fabs(rt) >= 0x1p-126 && fabs(rt) <= 0x1p126) || !(fabsf(sum) <= 3.0e38f);
   }
   auto body = [&](auto fastc) {
     constexpr bool FAST = decltype(fastc)::value;
@@ -135,7 +142,8 @@ __device__ __forceinline__ bool face_eval(const Stage2Args& a, const Offs& o, lo
     [[maybe_unused]] const C_ rtC = (C_)rt, rrC = (C_)rr, ptC = (C_)ptot, ebC = (C_)eb, eC = (C_)e, rhoC = (C_)rho, rhobC = (C_)rhob;
     auto by_rtC = [&](C_ n) {
       if constexpr (sizeof(S) == 8) return by_rt(n);
-      else return qdiv<true>(n, rtC, rrC);
+      else if constexpr (FAST) return qdiv<true>(n, rtC, rrC);
+      else return n / rtC;
     };
     C_ s1 = C_(0), s2 = C_(0);
 #pragma unroll
@@ -186,11 +194,11 @@ __device__ __forceinline__ bool face_eval(const Stage2Args& a, const Offs& o, lo
       }
     }
   };
-  if (sizeof(S) == 8 && (bad || a.quiet))
+  if (bad || (sizeof(S) == 8 && a.quiet))
     body(std::false_type{});
   else
     body(std::true_type{});
-  return bad;
+  return sizeof(S) == 8 && bad;
 }
 
 // k_face body at local cell c: the derived fields and every flux into D and F

@@ -8,7 +8,7 @@ and huge fields beside ordinary ones."""
 import numpy as np
 import pytest
 
-from sac_b200 import abi, problems
+from sac_b200 import abi, params, problems
 
 import _util
 
@@ -92,3 +92,29 @@ def test_split_sweep_and_variable_list_equal_the_oracle(nx, ndir):
     for kw in (dict(idimmin=2, idimmax=2), dict(iws=[1, 2, ndir + 2])):
         got, want = _one_step(P, **kw)
         np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("what", ["vacuum", "inf"])
+@pytest.mark.parametrize("nx,ndir", SHAPES)
+def test_fp32_infinities_are_the_quotients_own(nx, ndir, what):
+    """FP32 storage: where a cell has no density or an infinite momentum, a stage's NaN
+    and its infinities lie where the oracle's divides put them."""
+    from oracle.oracle import Oracle
+
+    P = problems.random_problem(nx, ndir=ndir, seed=52, nu=0.0, typeadvance="onestep")
+    mid, rhob = tuple(n // 2 for n in P.w.shape[:-1]), problems.var_index(ndir)["rhob"]
+    if what == "vacuum":
+        P.w[mid][rhob], P.w[mid][0] = 1.0, -1.0
+    else:
+        P.w[mid][1] = np.inf
+    o = _util.start(Oracle, P)
+    P.params.precision = params.PREC_FP32
+    c = _util.start(abi.Context, P)
+    got, want = [], []
+    for x, out in ((c, got), (o, want)):
+        x.advect(1e-3, 0.0, 0)
+        out.append(_util.mesh(P, x.download())[..., : 2 * ndir + 2])
+        x.close()
+    assert not np.isfinite(want[0]).all() and np.isfinite(want[0]).any()
+    np.testing.assert_array_equal(np.isnan(got[0]), np.isnan(want[0]))
+    np.testing.assert_array_equal(np.isinf(got[0]), np.isinf(want[0]))
