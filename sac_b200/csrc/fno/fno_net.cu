@@ -1026,12 +1026,17 @@ int backward(sac_fno* n, const bf16* dy) {
     d.err = n->errw;
     GK(d);
   }
+  // where the rows fit the row kernel, a layer's pointwise product, transposed transform
+  // along f, GELU' and the transform along f that the layer below starts with are one
+  // launch: it reads dz once instead of twice and keeps the sum of the two products in
+  // TMEM (at 16 samples of 256 x 256 the GEMMs wrote and read 134 MB of it in FP32)
+  const bool rows = row_ok(n);
   for (int l = n->L - 1; l >= 0; --l) {
     const bf16* v = n->act[l];
     bf16* dzl = n->dz;  // gradient w.r.t. z_l
     if ((rc = wgrad(n, dzl, W, v, W, gw + n->sW[l].off, B))) return rc;
     if ((rc = bias_grad(n, dzl, W, gw + n->sWb[l].off, B))) return rc;
-    {  // pointwise path: dvacc[b][i][p] = sum_o W[o][i] dz[b][o][p]
+    if (!rows) {  // pointwise path: dvacc[b][i][p] = sum_o W[o][i] dz[b][o][p]
       GemmDesc d = gd((int)P, W, W, B);
       a_chanfirst(d, dzl, W, P);
       d.b = n->wb + n->sW[l].off;
@@ -1042,7 +1047,8 @@ int backward(sac_fno* n, const bf16* dy) {
       d.err = n->errw;
       GK(d);
     }
-    {  // B5: dY[(b,o)][j'][s] = sum_f dz[(b,o,s)][f] Hy[f][j']
+    const bool from_row = rows && l < n->L - 1;  // dY came with dz, as T[b][s][o][j']
+    if (!from_row) {  // B5: dY[(b,o)][j'][s] = sum_f dz[(b,o,s)][f] Hy[f][j']
       GemmDesc d = gd(B * W * S, kJ, F);
       d.a = dzl;
       d.a_m0 = F;
@@ -1059,7 +1065,9 @@ int backward(sac_fno* n, const bf16* dy) {
       d.err = n->errw;
       GK(d);
     }
-    {  // B4: dP[(b,o),j'][r] = sum_s dY[(b,o),j'][s] Fx[r][s]  (rows r)
+    if (from_row) {
+      if ((rc = dft_s(n, n->dyt, n->dpt, B))) return rc;
+    } else {  // B4: dP[(b,o),j'][r] = sum_s dY[(b,o),j'][s] Fx[r][s]  (rows r)
       GemmDesc d = gd(kR, B * W * kJ, S);
       d.a = n->Fx;
       d.a_m0 = S;
@@ -1085,6 +1093,28 @@ int backward(sac_fno* n, const bf16* dy) {
                                                  n->dzt, gw + n->sRr[l].off, gw + n->sRi[l].off, B, W, n->m2);
       }
       FK(cudaGetLastError());
+    }
+    if (rows) {  // B2 as dT[(b,c)][s][j]; then dz_{l-1} = (W^T dz + Fy^T dT) GELU'(z_{l-1}) and its dY
+      if ((rc = idft_s(n, n->dzt, n->dtp, B))) return rc;
+      RowArgs a = row_args(n, B);
+      a.in = dzl;
+      a.w = n->wb + n->sW[l].off;  // W[o][i]: n = i, k = o
+      a.w_n = 1;
+      a.w_k = W;
+      a.h = n->FyT;
+      a.y = n->dtp;
+      a.out = n->dz2;
+      if (l > 0) {
+        a.pre = n->pre[l - 1];
+        a.g = n->HyT;
+        a.t = n->dyt;
+        rc = row_launch<32, true, ACT_GELU_GRAD, true, true>(n, a);
+      } else {
+        rc = row_launch<32, true, ACT_NONE, false, false>(n, a);
+      }
+      if (rc) return rc;
+      std::swap(n->dz, n->dz2);
+      continue;
     }
     {  // B2: dT[(b,c),j][s] = sum_r dZ[(b,c),j][r] Fx[r][s]  (rows s)
       GemmDesc d = gd(S, B * W * kJ, kR);
@@ -1320,7 +1350,7 @@ int sac_fno_create(const sac_fno_config* cfg, sac_fno** out) {
   FK(cudaMalloc(&n->dpt, sizeof(float) * B * W * kJ * kR));
   FK(cudaMalloc(&n->yb, sizeof(bf16) * B * W * n->S * kJ));
   FK(cudaMalloc(&n->spec, sizeof(float) * BWP));
-  FK(cudaMalloc(&n->dvacc, sizeof(float) * BWP));
+  if (!row_ok(n)) FK(cudaMalloc(&n->dvacc, sizeof(float) * BWP));
   FK(cudaMalloc(&n->dz, sizeof(bf16) * BWP));
   FK(cudaMalloc(&n->dz2, sizeof(bf16) * BWP));
   FK(cudaMalloc(&n->scal, sizeof(float) * 4));

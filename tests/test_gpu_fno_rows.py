@@ -72,3 +72,32 @@ def test_unaligned_buffers_give_the_same():
         assert torch.equal(a, b)
     # FP32 sums of 48384 squares in another order: n^0.5 * 2^-24 relative, with room
     assert abs(out[0][3] - out[1][3]) <= 1e-4 * abs(out[1][3])
+
+
+@pytest.mark.parametrize("S,F,B", [(56, 56, 1), (56, 128, 1), (64, 136, 3), (104, 248, 2), (64, 256, 1), (56, 264, 1)])
+def test_gradients_match_the_oracle(S, F, B):
+    """Every gradient group within the BF16 network's bound (5e-2 relative L2)."""
+    net, lay = _net(S, F, B), fno_ref.Layout(32, 4, 16, 6, 128)
+    g = torch.Generator().manual_seed(10)
+    x = torch.randn(B, 16, S, F, generator=g).to(torch.bfloat16)
+    dy = torch.zeros(B, net.cpad, S, F)
+    dy[:, :6] = torch.randn(B, 6, S, F, generator=g)
+    dy = dy.to(torch.bfloat16)
+    xd, dyd, y = x.cuda(), dy.cuda(), torch.zeros(B, 6, S, F, device="cuda")
+    torch.cuda.synchronize()
+    net.zero_grad()
+    net.forward(xd.data_ptr(), y.data_ptr(), B)
+    net.backward(dyd.data_ptr())
+    net.check()
+    got = net.get_grads().astype(np.float64)
+    theta = net.get_params().astype(np.float64)
+    for name, (o, n) in lay.segs.items():
+        if not name.endswith("b") and not (name[-1].isdigit() and name.startswith("Wb")):
+            theta[o:o + n] = fno_ref.bf16_round(theta[o:o + n])
+    _, tape = fno_ref.forward(lay, theta, x.double().numpy())
+    want = fno_ref.backward(lay, theta, tape, dy[:, :6].double().numpy())
+    for name, (o, n) in lay.segs.items():
+        if name in ("Q2", "Q2b"):
+            n = 6 * (128 if name == "Q2" else 1)
+        err = np.linalg.norm(got[o:o + n] - want[o:o + n]) / np.linalg.norm(want[o:o + n])
+        assert err < 5e-2, (name, err)
