@@ -31,6 +31,7 @@
 #include "fno_host.h"
 #include "fno_proj.cuh"
 #include "fno_row.cuh"
+#include "fno_wgrad.cuh"
 #include "sac_fno.h"
 
 using namespace fno;
@@ -991,6 +992,27 @@ int bias_grad(sac_fno* n, const bf16* d, int C, float* out, int B) {
 }
 
 // dy: [B][cpad][P] bf16 (gradient of the loss w.r.t. y; padding channels zero)
+// both gradients of a layer with 32 output and C = 32 or 16 input channels in one pass
+// where the rows allow it and `in` is on a 16-byte boundary; else wgrad and bias_grad
+int layer_grad(sac_fno* n, const bf16* dz, const bf16* in, int C, float* gw, float* gb, int B) {
+  if (!row_ok(n) || (uintptr_t)in & 15) {
+    int rc = wgrad(n, dz, n->W, in, C, gw, B);
+    return rc ? rc : bias_grad(n, dz, n->W, gb, B);
+  }
+  auto go = [&](auto Cc) -> int {
+    constexpr int K = decltype(Cc)::value, smem = WgradSmem<K>::BYTES;
+    FK(cudaFuncSetAttribute(k_wgrad<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    int nsm = 148;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, n->cfg.device);
+    const long ntask = (long)B * (n->S / 4);
+    const WgradArgs a{dz, in, gw, gb, B, n->S, n->F, n->errw, n->wait_tries};
+    k_wgrad<K><<<(unsigned)std::min<long>(ntask, nsm), kWgThreads, smem, n->st>>>(a);
+    FK(cudaGetLastError());
+    return 0;
+  };
+  return C == kRowN ? go(std::integral_constant<int, kRowN>{}) : go(std::integral_constant<int, 16>{});
+}
+
 int backward(sac_fno* n, const bf16* dy) {
   const int B = n->Blast, S = n->S, F = n->F, W = n->W, H = n->H, cpad = n->cpad;
   const long P = n->P;
@@ -1034,8 +1056,7 @@ int backward(sac_fno* n, const bf16* dy) {
   for (int l = n->L - 1; l >= 0; --l) {
     const bf16* v = n->act[l];
     bf16* dzl = n->dz;  // gradient w.r.t. z_l
-    if ((rc = wgrad(n, dzl, W, v, W, gw + n->sW[l].off, B))) return rc;
-    if ((rc = bias_grad(n, dzl, W, gw + n->sWb[l].off, B))) return rc;
+    if ((rc = layer_grad(n, dzl, v, W, gw + n->sW[l].off, gw + n->sWb[l].off, B))) return rc;
     if (!rows) {  // pointwise path: dvacc[b][i][p] = sum_o W[o][i] dz[b][o][p]
       GemmDesc d = gd((int)P, W, W, B);
       a_chanfirst(d, dzl, W, P);
@@ -1158,9 +1179,7 @@ int backward(sac_fno* n, const bf16* dy) {
     std::swap(n->dz, n->dz2);  // dz now holds the gradient w.r.t. z_{l-1} (or v_0)
   }
   // lift: v0 = Pw x + pb
-  if ((rc = wgrad(n, n->dz, W, n->xin, n->cin, gw + n->sP.off, B))) return rc;
-  if ((rc = bias_grad(n, n->dz, W, gw + n->sPb.off, B))) return rc;
-  return 0;
+  return layer_grad(n, n->dz, n->xin, n->cin, gw + n->sP.off, gw + n->sPb.off, B);
 }
 
 void make_tables(int S, int F, int m1, int m2, std::vector<float>& Fy, std::vector<float>& Fx,
