@@ -379,6 +379,9 @@ __global__ void k_sumsq(const float* __restrict__ g, long n, float* out) {
 
 // loss = mean (y - t)^2 over the first cout channels; dy = 2 (y - t) / n as BF16
 // in a buffer of cpad >= cout channels (the padding channels are zeroed)
+// The loss is one atomic per warp: FP32 additions to a running total round by the size
+// of each addend, whatever their order, so another grouping (one per block, 67 -> 10 us
+// for 16 samples of 256 x 256) moved it by up to 2e-5, as much as FP32 results may differ
 __global__ void k_mse(const float* __restrict__ y, const bf16* __restrict__ t, bf16* __restrict__ dy, float* loss,
                       int B, int cout, int cpad, long P, float inv_n) {
   float s = 0.f;
@@ -396,46 +399,6 @@ __global__ void k_mse(const float* __restrict__ y, const bf16* __restrict__ t, b
   }
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) atomicAdd(loss, s * inv_n);
-}
-
-// the same with 8 pixels of one channel per thread and one atomic per block (P a
-// multiple of 8, 16-byte aligned y, t and dy): 16 samples of 256 x 256, 67 -> 10 us
-__global__ void __launch_bounds__(256) k_mse8(const float* __restrict__ y, const bf16* __restrict__ t,
-                                              bf16* __restrict__ dy, float* loss, int nbc, int cout, int cpad, int P8,
-                                              float inv_n) {
-  __shared__ float sh[8];
-  float s = 0.f;
-  for (int bc = blockIdx.y; bc < nbc; bc += gridDim.y) {
-    const int c = bc % cpad, b = bc / cpad;
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < P8; q += gridDim.x * blockDim.x) {
-      float g[8] = {};
-      if (c < cout) {
-        const long o = ((long)b * cout + c) * P8 + q;
-        const float4 u0 = reinterpret_cast<const float4*>(y)[2 * o], u1 = reinterpret_cast<const float4*>(y)[2 * o + 1];
-        const uint4 tv = reinterpret_cast<const uint4*>(t)[o];
-        const bf16* te = reinterpret_cast<const bf16*>(&tv);
-        const float v[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float e = v[k] - __bfloat162float(te[k]);
-          s += e * e;
-          g[k] = 2.f * e * inv_n;
-        }
-      }
-      __nv_bfloat162 o2[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) o2[k] = __floats2bfloat162_rn(g[2 * k], g[2 * k + 1]);
-      reinterpret_cast<uint4*>(dy)[(long)bc * P8 + q] = *reinterpret_cast<const uint4*>(o2);
-    }
-  }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    s = 0.f;
-    for (int w = 0; w < 8; ++w) s += sh[w];
-    atomicAdd(loss, s * inv_n);
-  }
 }
 
 // network input x[b][c][s][f] (bf16, cin channels):
@@ -1518,12 +1481,7 @@ int sac_fno_backward(sac_fno* n, const void* dy) {
 int sac_fno_mse(sac_fno* n, const float* y, const void* target, void* dy, float* loss, int B) {
   if (!n || !y || !target || !dy || !loss) return fail(n, "sac_fno_mse: null argument");
   const long tot = (long)B * n->cout * n->P;
-  if (aligned16p(y) && aligned16p(target) && aligned16p(dy))
-    k_mse8<<<grid_rows((long)B * n->cpad, n->P / 8), 256, 0, n->st>>>(y, (const bf16*)target, (bf16*)dy, loss,
-                                                                     B * n->cpad, n->cout, n->cpad, (int)(n->P / 8),
-                                                                     1.0f / (float)tot);
-  else
-    k_mse<<<grid_for((long)B * n->cpad * n->P), 256, 0, n->st>>>(y, (const bf16*)target, (bf16*)dy, loss, B,
+  k_mse<<<grid_for((long)B * n->cpad * n->P), 256, 0, n->st>>>(y, (const bf16*)target, (bf16*)dy, loss, B,
                                                                n->cout, n->cpad, n->P, 1.0f / (float)tot);
   FK(cudaGetLastError());
   return 0;

@@ -41,7 +41,7 @@ def test_forward_matches_the_oracle(S, F, B):
 
 
 def test_unaligned_buffers_give_the_same():
-    """features, apply and mse with buffers off the 16-byte boundary take the scalar
+    """features and apply with buffers off the 16-byte boundary take the scalar
     kernels: the same values (the loss up to the order of its sum)."""
     S, F, B = 56, 72, 2
     net = _net(S, F, B)
@@ -74,7 +74,8 @@ def test_unaligned_buffers_give_the_same():
     assert abs(out[0][3] - out[1][3]) <= 1e-4 * abs(out[1][3])
 
 
-@pytest.mark.parametrize("S,F,B", [(56, 56, 1), (56, 128, 1), (64, 136, 3), (104, 248, 2), (64, 256, 1), (56, 264, 1)])
+@pytest.mark.parametrize("S,F,B", [(56, 56, 1), (56, 128, 1), (64, 136, 3), (200, 120, 5), (104, 248, 2), (64, 256, 1),
+                                   (56, 264, 1)])
 def test_gradients_match_the_oracle(S, F, B):
     """Every gradient group within the BF16 network's bound (5e-2 relative L2)."""
     net, lay = _net(S, F, B), fno_ref.Layout(32, 4, 16, 6, 128)
