@@ -955,25 +955,36 @@ int bias_grad(sac_fno* n, const bf16* d, int C, float* out, int B) {
 }
 
 // dy: [B][cpad][P] bf16 (gradient of the loss w.r.t. y; padding channels zero)
-// both gradients of a layer with 32 output and C = 32 or 16 input channels in one pass
-// where the rows allow it and `in` is on a 16-byte boundary; else wgrad and bias_grad
-int layer_grad(sac_fno* n, const bf16* dz, const bf16* in, int C, float* gw, float* gb, int B) {
-  if (!row_ok(n) || (uintptr_t)in & 15) {
-    int rc = wgrad(n, dz, n->W, in, C, gw, B);
-    return rc ? rc : bias_grad(n, dz, n->W, gb, B);
+// one k_wgrad launch: persistent, one CTA per SM
+template <int R, int C, bool TR>
+int wgrad_launch(sac_fno* n, const bf16* d, const bf16* in, float* gw, float* gb, int B) {
+  constexpr int smem = WgradSmem<R, C>::BYTES;
+  auto* k = k_wgrad<R, C, TR>;
+  FK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  int nsm = 148;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, n->cfg.device);
+  const long ntask = (long)B * (n->S / WgradSmem<R, C>::ROWS);
+  const WgradArgs a{d, in, gw, gb, B, n->S, n->F, n->errw, n->wait_tries};
+  k<<<(unsigned)std::min<long>(ntask, nsm), kWgThreads, smem, n->st>>>(a);
+  FK(cudaGetLastError());
+  return 0;
+}
+
+// both gradients of a product with R outputs and C inputs per pixel, in one pass where
+// k_wgrad has the shape, the rows allow it and the operands are on 16-byte boundaries
+int layer_grad(sac_fno* n, const bf16* d, int R, const bf16* in, int C, float* gw, float* gb, int B) {
+  int rc;
+  if (row_ok(n) && (((uintptr_t)d | (uintptr_t)in) & 15) == 0) {
+    if (R == 32 && C == 32) return wgrad_launch<32, 32, false>(n, d, in, gw, gb, B);
+    if (R == 32 && C == 16) return wgrad_launch<32, 16, false>(n, d, in, gw, gb, B);
+    if (R == 128 && C == 32) return wgrad_launch<128, 32, false>(n, d, in, gw, gb, B);
+    if (R == 8 && C == 128) {  // the wide operand fills the tile's rows
+      rc = wgrad_launch<128, 8, true>(n, in, d, gw, nullptr, B);
+      return rc ? rc : bias_grad(n, d, R, gb, B);
+    }
   }
-  auto go = [&](auto Cc) -> int {
-    constexpr int K = decltype(Cc)::value, smem = WgradSmem<K>::BYTES;
-    FK(cudaFuncSetAttribute(k_wgrad<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    int nsm = 148;
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, n->cfg.device);
-    const long ntask = (long)B * (n->S / 4);
-    const WgradArgs a{dz, in, gw, gb, B, n->S, n->F, n->errw, n->wait_tries};
-    k_wgrad<K><<<(unsigned)std::min<long>(ntask, nsm), kWgThreads, smem, n->st>>>(a);
-    FK(cudaGetLastError());
-    return 0;
-  };
-  return C == kRowN ? go(std::integral_constant<int, kRowN>{}) : go(std::integral_constant<int, 16>{});
+  rc = wgrad(n, d, R, in, C, gw, B);
+  return rc ? rc : bias_grad(n, d, R, gb, B);
 }
 
 int backward(sac_fno* n, const bf16* dy) {
@@ -983,8 +994,7 @@ int backward(sac_fno* n, const bf16* dy) {
   // y = Q2 h + q2b
   int rc;
   // dy holds cpad channels (the ones past cout are zero, as are those rows of Q2)
-  if ((rc = wgrad(n, dy, cpad, n->h, H, gw + n->sQ2.off, B))) return rc;
-  if ((rc = bias_grad(n, dy, cpad, gw + n->sQ2b.off, B))) return rc;
+  if ((rc = layer_grad(n, dy, cpad, n->h, H, gw + n->sQ2.off, gw + n->sQ2b.off, B))) return rc;
   {  // dhpre[b][q][p] = GELU'(hpre) * sum_k Q2[k][q] dy[b][k][p]
     GemmDesc d = gd((int)P, H, cpad, B);
     a_chanfirst(d, dy, cpad, P);
@@ -998,8 +1008,7 @@ int backward(sac_fno* n, const bf16* dy) {
     d.err = n->errw;
     GK(d);
   }
-  if ((rc = wgrad(n, n->dhpre, H, n->act[n->L], W, gw + n->sQ1.off, B))) return rc;
-  if ((rc = bias_grad(n, n->dhpre, H, gw + n->sQ1b.off, B))) return rc;
+  if ((rc = layer_grad(n, n->dhpre, H, n->act[n->L], W, gw + n->sQ1.off, gw + n->sQ1b.off, B))) return rc;
   {  // dz_{L-1}[b][o][p] = sum_q Q1[q][o] dhpre[b][q][p]   (no activation after the last layer)
     GemmDesc d = gd((int)P, W, H, B);
     a_chanfirst(d, n->dhpre, H, P);
@@ -1019,7 +1028,7 @@ int backward(sac_fno* n, const bf16* dy) {
   for (int l = n->L - 1; l >= 0; --l) {
     const bf16* v = n->act[l];
     bf16* dzl = n->dz;  // gradient w.r.t. z_l
-    if ((rc = layer_grad(n, dzl, v, W, gw + n->sW[l].off, gw + n->sWb[l].off, B))) return rc;
+    if ((rc = layer_grad(n, dzl, W, v, W, gw + n->sW[l].off, gw + n->sWb[l].off, B))) return rc;
     if (!rows) {  // pointwise path: dvacc[b][i][p] = sum_o W[o][i] dz[b][o][p]
       GemmDesc d = gd((int)P, W, W, B);
       a_chanfirst(d, dzl, W, P);
@@ -1142,7 +1151,7 @@ int backward(sac_fno* n, const bf16* dy) {
     std::swap(n->dz, n->dz2);  // dz now holds the gradient w.r.t. z_{l-1} (or v_0)
   }
   // lift: v0 = Pw x + pb
-  return layer_grad(n, n->dz, n->xin, n->cin, gw + n->sP.off, gw + n->sPb.off, B);
+  return layer_grad(n, n->dz, W, n->xin, n->cin, gw + n->sP.off, gw + n->sPb.off, B);
 }
 
 void make_tables(int S, int F, int m1, int m2, std::vector<float>& Fy, std::vector<float>& Fx,
