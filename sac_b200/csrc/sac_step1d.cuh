@@ -67,6 +67,9 @@ __global__ void __cluster_dims__(kStep1dCtas, 1, 1) __launch_bounds__(kStep1dThr
   auto slot = [](int iw) { return iw < B0 + 1 ? iw : iw - 1; };  // b_1 (variable B0 + 1) has no flux
   long ns[3];
   ghost_slabs(g, ns);
+  // a CTA's shared memory may be written by the others only once it is known to have
+  // started: arrive here, wait before the first write (stage 0), behind its k_face
+  cluster.barrier_arrive();
 #pragma unroll 1
   for (int s = 0; s < 4; ++s) {
     const Stage2Args& a = p.st[s];
@@ -89,6 +92,7 @@ __global__ void __cluster_dims__(kStep1dCtas, 1, 1) __launch_bounds__(kStep1dThr
       if (mesh) cm = (cc != cc || cm != cm) ? __longlong_as_double(0x7ff8000000000000ll) : fmax(cm, cc);
     }
     double ct = 0.0;
+    if (s == 0) cluster.barrier_wait();
     if (a.visc_on) {
       cm = block_max_all(cm, sh);
       if (tid < kStep1dCtas) *cluster.map_shared_rank(&ct_part[rank], tid) = cm;
