@@ -177,7 +177,9 @@ cudaError_t launch_step1d(const Step1dArgs& p0, cudaStream_t st) {
   const unsigned nt = (unsigned)std::min(kStep1dThreads, (m + 31) / 32 * 32);
   auto go = [&](auto NR) -> cudaError_t {
     auto* k = k_step1d<decltype(NR)::value, S>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    // the kernel's own limit, not this grid's size: host threads with grids of other
+    // sizes share the attribute
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kStep1dSmem);
     if (e != cudaSuccess) return e;
     k<<<kStep1dCtas, nt, smem, st>>>(p);
     return cudaGetLastError();
