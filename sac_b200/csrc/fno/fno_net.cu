@@ -56,6 +56,7 @@ __global__ void k_f2bf(bf16* dst, const float* src, long n) {
 // Shared memory: R of the 8 modes as [i][o][j] and U as [(b,i)][j], j = q - q0
 // fastest, so that a warp's reads of both are conflict-free.
 constexpr int kMixQ = 8;
+constexpr size_t kMixSmem = 227 * 1024;  // the mode mixing's dynamic shared memory at most (it has no static)
 __global__ void __launch_bounds__(256) k_mix_fwd(const float* __restrict__ zt, const bf16* __restrict__ Rr,
                                                  const bf16* __restrict__ Ri, bf16* __restrict__ pt, int B, int W,
                                                  int m2) {
@@ -1252,22 +1253,23 @@ int sac_fno_create(const sac_fno_config* cfg, sac_fno** out) {
     delete n;
     return fail(nullptr, "sac_fno_create: no device");
   }
-  {  // the grouped forward mode mixing holds R and U of 8 modes for the whole batch
+  {  // the mode mixing's shared memory follows max_batch; the kernels' limit is set to
+     // the same value by every network, since the attribute belongs to the process and a
+     // smaller network would lower it for a larger one
+    auto fits = [](auto* k, size_t bytes) {
+      const bool ok = bytes <= kMixSmem && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                                (int)kMixSmem) == cudaSuccess;
+      cudaGetLastError();  // a refused attribute leaves the per-mode form
+      return ok;
+    };
+    // the grouped forward mode mixing holds R and U of 8 modes for the whole batch
     const size_t mix = sizeof(float) * kMixQ * (2 * (size_t)n->W * n->W + 2 * (size_t)n->Bmax * n->W);
-    n->mix_grouped = mix <= 227 * 1024 && (2 * n->m1) % kMixQ == 0 &&
-                     cudaFuncSetAttribute(k_mix_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mix) ==
-                         cudaSuccess;
-    cudaGetLastError();  // a refused attribute leaves the per-mode form
+    n->mix_grouped = (2 * n->m1) % kMixQ == 0 && fits(k_mix_fwd, mix);
     // the grouped backward holds R, U and G of 8 modes for the training batch
-    const size_t mb = std::min<size_t>(227 * 1024, sizeof(float) * kMixQ *
-                                                       (2 * (size_t)n->W * n->W + 4 * (size_t)n->Bmax * n->W));
-    if ((2 * n->m1) % kMixQ == 0 &&
-        cudaFuncSetAttribute(k_mix_bwd_g, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mb) == cudaSuccess)
-      n->mix_bwd_max = mb;
-    cudaGetLastError();
+    const size_t mb = std::min(kMixSmem, sizeof(float) * kMixQ * (2 * (size_t)n->W * n->W + 4 * (size_t)n->Bmax * n->W));
+    if ((2 * n->m1) % kMixQ == 0 && fits(k_mix_bwd_g, mb)) n->mix_bwd_max = mb;
     const size_t one = sizeof(float) * (2 * (size_t)n->W * n->W + 2 * (size_t)n->Bmax * n->W);
-    if (!n->mix_grouped &&
-        cudaFuncSetAttribute(k_mix_fwd_mode, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)one) != cudaSuccess) {
+    if (!n->mix_grouped && !fits(k_mix_fwd_mode, one)) {
       cudaStreamDestroy(n->st);
       delete n;
       return fail(nullptr, "sac_fno_create: width and max_batch too large for the mode mixing's shared memory");

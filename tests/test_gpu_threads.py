@@ -50,3 +50,33 @@ def test_1d_grids_of_different_sizes_in_their_threads():
     assert not err, err
     for k in range(4):
         np.testing.assert_array_equal(out[k], alone[large if k == 3 else small])
+
+
+@pytest.mark.parametrize("width,B", [(32, 32), (64, 64)])
+def test_a_smaller_network_beside_a_larger_one(width, B):
+    """The mode mixing's shared memory follows max_batch: a network of one sample made
+    later leaves the larger one its launches."""
+    torch = pytest.importorskip("torch")
+    from sac_b200 import fno_abi
+
+    S = F = 56
+    net = fno_abi.Net(S=S, F=F, width=width, layers=1, max_batch=B, seed=5)
+    x = torch.randn(B, 16, S, F, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).cuda()
+    dy = torch.zeros(B, net.cpad, S, F, dtype=torch.bfloat16, device="cuda")
+    dy[:, :6] = 1e-3
+    y = [torch.zeros(B, 6, S, F, device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    grads = []
+    for k in range(2):
+        net.zero_grad()
+        net.forward(x.data_ptr(), y[k].data_ptr(), B)
+        if width == 32:  # the wider network trains on smaller batches only
+            net.backward(dy.data_ptr())
+        net.check()
+        grads.append(net.get_grads())
+        other = fno_abi.Net(S=S, F=F, width=width, layers=1, max_batch=1, seed=6)
+    assert torch.equal(y[0], y[1])
+    # sums of atomic additions, in another order from run to run
+    assert np.linalg.norm(grads[0] - grads[1]) <= 1e-4 * np.linalg.norm(grads[0]) + 1e-30
+    other.close()
+    net.close()
