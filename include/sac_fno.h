@@ -125,6 +125,9 @@ int sac_fno_check(sac_fno* n, int reset);
 /* wait_tries of every GEMM the network launches (see sac_fno_gemm_desc; 0 =
  * default, -1 = give up at once, for testing the time-out report) */
 int sac_fno_set_wait_tries(sac_fno* n, int tries);
+/* the same for one wait alone: the row kernel's, for the product with the next layer's
+ * transform (0 = as the others) */
+int sac_fno_set_t_wait_tries(sac_fno* n, int tries);
 
 #ifdef __cplusplus
 }

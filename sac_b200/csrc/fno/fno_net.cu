@@ -544,6 +544,7 @@ struct sac_fno {
   float *spec = nullptr, *dvacc = nullptr, *dpt = nullptr, *scal = nullptr;
   int* errw = nullptr;
   int wait_tries = 0;  // GemmDesc::wait_tries of every launch (0: default bound)
+  int t_wait_tries = 0;  // RowArgs::t_wait_tries
 };
 
 namespace {
@@ -628,6 +629,7 @@ RowArgs row_args(sac_fno* n, int B) {
   a.F = n->F;
   a.err = n->errw;
   a.wait_tries = n->wait_tries;
+  a.t_wait_tries = n->t_wait_tries;
   return a;
 }
 
@@ -1569,6 +1571,12 @@ int sac_fno_check(sac_fno* n, int reset) {
 int sac_fno_set_wait_tries(sac_fno* n, int tries) {
   if (!n) return 1;
   n->wait_tries = tries < 0 ? -1 : tries;
+  return 0;
+}
+
+int sac_fno_set_t_wait_tries(sac_fno* n, int tries) {
+  if (!n) return 1;
+  n->t_wait_tries = tries < 0 ? -1 : tries;
   return 0;
 }
 

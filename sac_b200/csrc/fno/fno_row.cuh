@@ -47,6 +47,7 @@ struct RowArgs {
   int B, S, F;
   int* err;
   int wait_tries;
+  int t_wait_tries;  // of the wait for the product with G alone (the same meaning)
 };
 
 constexpr int kRowN = 32, kRowJ = 48, kRowF = 256, kRowThreads = 512;
@@ -132,6 +133,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_row(const __grid_constant__ 
   const uint32_t tmem = tmem_sh;
   const uint32_t id1 = umma_idesc(kRowN, 1, 0), id2 = umma_idesc(kRowN, 0, 0), idt = umma_idesc(kRowJ, 1, 0);
   const int tries = a.wait_tries == 0 ? kWaitTries : (a.wait_tries < 0 ? 0 : a.wait_tries);
+  const int t_tries = a.t_wait_tries == 0 ? tries : (a.t_wait_tries < 0 ? 0 : a.t_wait_tries);
 
   // this CTA's rows: tasks of 4 rows, blockIdx.x, + gridDim.x, ...
   const int S4 = S / 4, ntask = a.B * S4;
@@ -204,7 +206,8 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_row(const __grid_constant__ 
   int t_done = 0;    // ... and stored
   // T of the task whose product was issued last: row m = (s, n) of the accumulator
   auto store_t = [&]() {
-    if (!mbar_wait(&bar_t, (uint32_t)(t_done & 1), tries)) {
+    // one outcome per warp: the loads below need all its lanes, together
+    if (!__all_sync(0xffffffffu, mbar_wait(&bar_t, (uint32_t)(t_done & 1), t_tries))) {
       ok = false;
       return;
     }
@@ -305,7 +308,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_row(const __grid_constant__ 
       // the product of the task before has read the staged rows, and its accumulator is
       // free for the next one
       if (pe.r == 0 && t_issued > t_done && ok) store_t();
-      if (live) {  // (f/8 * 16 + (r*4 + n/8))*128 + f%8*16
+      if (live && ok) {  // (f/8 * 16 + (r*4 + n/8))*128 + f%8*16
         uint8_t* d = smem + L::OUT + ((f >> 3) * 16 + (pe.r + w) * 4) * 128 + (f & 7) * 16;
 #pragma unroll
         for (int q = 0; q < 4; ++q)

@@ -130,9 +130,11 @@ def _bind_net(lib):
     lib.sac_fno_apply.argtypes = [VP, VP, VP, VP, ctypes.c_int, ctypes.c_int]
     lib.sac_fno_check.argtypes = [VP, ctypes.c_int]
     lib.sac_fno_set_wait_tries.argtypes = [VP, ctypes.c_int]
+    lib.sac_fno_set_t_wait_tries.argtypes = [VP, ctypes.c_int]
     for f in ("sac_fno_create", "sac_fno_param_layout", "sac_fno_init", "sac_fno_set_params", "sac_fno_get_params",
               "sac_fno_get_grads", "sac_fno_zero_grad", "sac_fno_forward", "sac_fno_infer", "sac_fno_backward", "sac_fno_mse",
-              "sac_fno_adam", "sac_fno_features", "sac_fno_apply", "sac_fno_check", "sac_fno_set_wait_tries"):
+              "sac_fno_adam", "sac_fno_features", "sac_fno_apply", "sac_fno_check", "sac_fno_set_wait_tries",
+              "sac_fno_set_t_wait_tries"):
         getattr(lib, f).restype = ctypes.c_int
     lib._net_bound = True
     return lib
@@ -224,6 +226,10 @@ class Net:
     def set_wait_tries(self, tries):
         """Bound of the tensor-core waits of every GEMM (0: default; -1: give up at once)."""
         self._c(self.lib.sac_fno_set_wait_tries(self.h, int(tries)))
+
+    def set_t_wait_tries(self, tries):
+        """The same for the row kernel's wait for its last product alone."""
+        self._c(self.lib.sac_fno_set_t_wait_tries(self.h, int(tries)))
 
     def close(self):
         if self.h:

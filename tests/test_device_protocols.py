@@ -23,3 +23,19 @@ def test_distributed_shared_memory_is_reached_after_a_cluster_barrier(name):
     wait = re.search(r"cluster\.(sync|barrier_wait)\(\)", src)
     assert wait and wait.start() < access
     assert src.count("barrier_arrive()") == src.count("barrier_wait()")
+
+
+@pytest.mark.parametrize("name", ["fno_gemm.cuh", "fno_proj.cuh", "fno_row.cuh", "fno_wgrad.cuh"])
+def test_a_bounded_wait_ends_alike_for_a_warp_before_it_loads_an_accumulator(name):
+    """tcgen05.ld is executed by all lanes of a warp together, and a wait with a bound may
+    end in time for some and not for others: a vote of the warp or of the block stands
+    between every such load and the wait before it."""
+    src = _code(os.path.join("fno", name))
+    # (a wait whose result is not used lets products drain, with no load behind it)
+    waits = [m.start() for m in re.finditer(r"(?<=!)mbar_wait\(|(?<=, )mbar_wait\(", src)]
+    loads = [m.start() for m in re.finditer(r"tcgen05\.ld\.", src)]
+    assert loads
+    for ld in loads:
+        wait = max(w for w in waits if w < ld)
+        line = src.rindex("\n", 0, wait)
+        assert re.search(r"__all_sync|__syncthreads_or", src[line:ld]), src[line:wait + 60]

@@ -102,3 +102,29 @@ def test_gradients_match_the_oracle(S, F, B):
             n = 6 * (128 if name == "Q2" else 1)
         err = np.linalg.norm(got[o:o + n] - want[o:o + n]) / np.linalg.norm(want[o:o + n])
         assert err < 5e-2, (name, err)
+
+
+@pytest.mark.parametrize("B", [1, 64])
+def test_the_transform_wait_running_out_is_reported(B):
+    """The wait for the product with G, which a CTA reaches after each task of four rows
+    (one task per CTA, and several): sac_fno_check returns 7, and the network gives what it
+    gave before once the default bound is back."""
+    from sac_b200 import fno_abi
+
+    S, F = 56, 72
+    net = _net(S, F, B)
+    x = torch.randn(B, 16, S, F, generator=torch.Generator().manual_seed(9)).to(torch.bfloat16).cuda()
+    y = [torch.zeros(B, 6, S, F, device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    net.infer(x.data_ptr(), y[0].data_ptr(), B)
+    net.check()
+    net.set_t_wait_tries(-1)
+    net.infer(x.data_ptr(), y[1].data_ptr(), B)
+    with pytest.raises(fno_abi.FnoError) as e:
+        net.check(reset=True)
+    assert "status 7" in str(e.value)
+    net.set_t_wait_tries(0)
+    net.infer(x.data_ptr(), y[1].data_ptr(), B)
+    net.check(reset=True)
+    assert torch.equal(y[0], y[1])
+    net.close()
