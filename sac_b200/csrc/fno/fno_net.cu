@@ -487,9 +487,11 @@ __global__ void __launch_bounds__(256) k_apply4(float* __restrict__ st, const fl
   }
 }
 
-// a grid of rows (y) times chunks (x) for n items of 256 threads each per row
+// a grid of rows (y) times chunks (x) for n items of 256 threads each per row; at least
+// one block, which has no row to do where a call has none
 dim3 grid_rows(long rows, long n) {
-  return dim3((unsigned)std::max<long>(1, std::min<long>((n + 255) / 256, 64)), (unsigned)std::min<long>(rows, 65535));
+  return dim3((unsigned)std::max<long>(1, std::min<long>((n + 255) / 256, 64)),
+              (unsigned)std::max<long>(1, std::min<long>(rows, 65535)));
 }
 bool aligned16p(const void* p) { return ((uintptr_t)p & 15) == 0; }
 

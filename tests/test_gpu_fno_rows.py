@@ -128,3 +128,20 @@ def test_the_transform_wait_running_out_is_reported(B):
     net.check(reset=True)
     assert torch.equal(y[0], y[1])
     net.close()
+
+
+def test_no_samples_and_no_state_channels_are_no_work():
+    """features and apply of no samples, and apply of no channels, leave everything as it is."""
+    S, F = 56, 72
+    net = _net(S, F, 1)
+    st, sc = torch.ones(6, S, F, device="cuda"), torch.ones(6, device="cuda")
+    x = torch.ones(16, S, F, dtype=torch.bfloat16, device="cuda")
+    torch.cuda.synchronize()
+    for bf16 in (False, True):
+        net.features(st.data_ptr(), bf16, sc.data_ptr(), sc.data_ptr(), 4, x.data_ptr(), 0, 6)
+    net.apply(st.data_ptr(), st.data_ptr(), sc.data_ptr(), 0, 6)
+    net.apply(st.data_ptr(), st.data_ptr(), sc.data_ptr(), 1, 0)
+    net.check()
+    torch.cuda.synchronize()
+    assert bool((st == 1).all()) and bool((x == 1).all())
+    net.close()
