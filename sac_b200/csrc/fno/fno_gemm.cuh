@@ -360,6 +360,7 @@ __global__ void __launch_bounds__(kThreads, BN <= 64 ? 4 : BN <= 128 ? 3 : 1) k_
     const long crow = m < d.M ? (long)zb * d.c_b + (long)(m / d.c_msplit) * d.c_m1 + (long)(m % d.c_msplit) * d.c_m0 : 0;
 #pragma unroll 1
     for (int cc = 0; cc < BN; cc += 16) {
+      __syncwarp();  // lanes past M skip the rest of a turn; the load needs the whole warp
       uint32_t v[16];
       const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)cc;
       asm volatile(

@@ -39,3 +39,11 @@ def test_a_bounded_wait_ends_alike_for_a_warp_before_it_loads_an_accumulator(nam
         wait = max(w for w in waits if w < ld)
         line = src.rindex("\n", 0, wait)
         assert re.search(r"__all_sync|__syncthreads_or", src[line:ld]), src[line:wait + 60]
+
+
+def test_the_gemm_epilogue_gathers_its_warp_before_each_load():
+    """The lanes of rows past M leave a turn of the column loop early; the next turn's load
+    needs them back."""
+    src = _code(os.path.join("fno", "fno_gemm.cuh"))
+    turn = src[src.index("cc < BN"):]
+    assert turn.index("__syncwarp()") < turn.index("tcgen05.ld") < turn.index("continue")
