@@ -100,6 +100,7 @@ struct sac_ctx {
   int itmin = 0;
   bool itmin_set = false;
   long kernel_launches = 0;
+  int general_kernels = 0;  // the last stage's update ran the general form's own kernels
   cudaStream_t own_stream = nullptr;
   // event profiling
   bool prof = false;
@@ -438,6 +439,7 @@ sac_status advect1_t(sac_ctx* c, const std::string& method, double qdt, int dmin
       Prof pr(c, SAC_K_STAGE);
       launch_update<S>(a, c->stream);
     }
+    c->general_kernels = g.ndim > 1 && c->nflags && (a.general || a.quiet) ? 1 : 0;
   } else if (base != out) {
     CK(cudaMemcpyAsync(out, base, c->es * g.np * g.ncell, cudaMemcpyDeviceToDevice, c->stream));
   }
@@ -1558,6 +1560,8 @@ sac_status sac_diag(sac_ctx* c, sac_diag_out* out) {
 
 // Number of kernels this library launched on the context (benchmark accounting).
 long sac_kernel_launches(const sac_ctx* c) { return c ? c->kernel_launches : 0; }
+// which kernels the last stage's update ran, for the tests of that choice (not in the header)
+int sac_general_kernels(const sac_ctx* c) { return c ? c->general_kernels : 0; }
 
 sac_status sac_set_stream(sac_ctx* c, void* stream) {
   if (!c) return SAC_ERR_ARG;

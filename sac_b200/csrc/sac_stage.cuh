@@ -343,6 +343,9 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
   using PR = Pairs<NDIM>;
   using T = S;
   constexpr int NP = 2 * NDIR + 2, E = NDIR + 1, B0 = NDIR + 1;
+  // (the quiet kernels branch: their divides leave nothing to issue ahead, and the loads
+  // held in registers spilled; part A 16 -> 0 bytes, B 112 -> 96)
+  constexpr bool SELECT = (OPT & OPT_QUIET) == 0;
   T numax = T(0);
   {
     // stencil fields at c and its neighbours (st); the cell's own global fields at cg
@@ -410,12 +413,12 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
       }
       if (FAST || ((a.iwmask >> E) & 1u)) {
         const S* vd = Df(1 + d);
-        // getptotal_bg, src/vacphys0.t.mhd:221
-        double bgs = 0.0;
+        if (SELECT || !z4[d]) {
+          // getptotal_bg, src/vacphys0.t.mhd:221
+          double bgs = 0.0;
 #pragma unroll
-        for (int C = 0; C < NDIR; ++C) bgs = bgs + __ldg(BG(2 + C) + cg) * __ldg(BG(2 + C) + cg);
-        const T fb = (T)((a.gamma - 1.0) * __ldg(BG(0) + cg) - 0.5 * (a.gamma - 2.0) * bgs);
-        if (FAST || !z4[d]) {
+          for (int C = 0; C < NDIR; ++C) bgs = bgs + __ldg(BG(2 + C) + cg) * __ldg(BG(2 + C) + cg);
+          const T fb = (T)((a.gamma - 1.0) * __ldg(BG(0) + cg) - 0.5 * (a.gamma - 2.0) * bgs);
           const T t = acc[E] - qdt * g4(vd, d) * fb;
           acc[E] = z4[d] ? acc[E] : t;
         }
@@ -458,7 +461,15 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
       for (int d = 0; d < NDIM; ++d)
         z1[d] = (a.zero1[d][0] && pos[d] == g.lo[d]) || (a.zero1[d][1] && pos[d] == g.hi[d]);
       auto over = [&](T n, int d) { return qdiv<FAST>(n, dxv[d], rxv[d]); };
-      auto zero_if = [](bool z, T v) { return z ? T(0) : v; };
+      // zero where z: selected after the arithmetic, or branched around it
+      auto zero_if = [](bool z, auto&& v) -> T {
+        if constexpr (SELECT) {
+          const T t = v();
+          return z ? T(0) : t;
+        } else {
+          return z ? T(0) : v();
+        }
+      };
       auto nus = [&](int ip, int k, int j, T dxk, T& nl, T& nr) {
         const S* Qp = QQ(ip);
         nr = ldt<TILE>(Qp, j) * dxk;
@@ -475,8 +486,8 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
           nus(pass == 0 ? PR::rho(k) : PR::e(k), k, c, dxv[k], nl, nr);
           numax = fmaxT(numax, fmaxT(nr, nl));
           const T qc = ldt<TILE>(q, c);
-          const T gL = zero_if(z1[k], over(qc - ldt<TILE>(q, c - st[k]), k));
-          const T gR = zero_if(z1[k], over(ldt<TILE>(q, c + st[k]) - qc, k));
+          const T gL = zero_if(z1[k], [&] { return over(qc - ldt<TILE>(q, c - st[k]), k); });
+          const T gR = zero_if(z1[k], [&] { return over(ldt<TILE>(q, c + st[k]) - qc, k); });
           const T tL = (nl + T(0)) * gL, tR = (nr + T(0)) * gR;
           acc[tgt] = acc[tgt] + over(tR - tL, k) * q2;
         }
@@ -496,8 +507,8 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
           nus(PR::v(l, k), k, c, dxk, nl, nr);
           numax = fmaxT(numax, fmaxT(nr, nl));
           const T qc = ldt<TILE>(q, c);
-          const T gL = zero_if(z1[k], over(qc - ldt<TILE>(q, c - sk), k));
-          const T gR = zero_if(z1[k], over(ldt<TILE>(q, c + sk) - qc, k));
+          const T gL = zero_if(z1[k], [&] { return over(qc - ldt<TILE>(q, c - sk), k); });
+          const T gR = zero_if(z1[k], [&] { return over(ldt<TILE>(q, c + sk) - qc, k); });
           const T tL = (nl + T(0)) * gL, tR = (nr + T(0)) * gR;
           const S* ml = W(1 + l);
           const T mc = ldt<TILE>(ml, c);
@@ -523,7 +534,7 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
               T H = T(0);
               const bool in = pl >= g.lo[l] && pl <= g.hi[l];  // nu vanishes outside the mesh
               if constexpr ((OPT & OPT_PRE) != 0) {
-                H = zero_if(!in, ldt<TILE>((const S*)a.fX[Cross<NDIM>::m(l, k)] + o.I, j));
+                H = zero_if(!in, [&] { return ldt<TILE>((const S*)a.fX[Cross<NDIM>::m(l, k)] + o.I, j); });
               } else {
                 if (in) {
                   T dxkj, rxkj;
@@ -537,8 +548,8 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
               Tm[sg] = ldt<TILE>(rtf, j) * H;
               Te[sg] = ldt<TILE>(W(1 + k), j) * H;
             }
-            const T tCm = zero_if(z1[l], over(Tm[1] - Tm[0], l) / T(2));
-            const T tCe = zero_if(z1[l], over(Te[1] - Te[0], l) / T(2));
+            const T tCm = zero_if(z1[l], [&] { return over(Tm[1] - Tm[0], l) / T(2); });
+            const T tCe = zero_if(z1[l], [&] { return over(Te[1] - Te[0], l) / T(2); });
             acc[1 + k] = acc[1 + k] + tCm * q2;
             acc[E] = acc[E] + tCe * q2;
           }
@@ -567,7 +578,7 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
               T Kv = T(0);
               const bool in = pl >= g.lo[l] && pl <= g.hi[l];
               if constexpr ((OPT & OPT_PRE) != 0) {
-                Kv = zero_if(!in, ldt<TILE>((const S*)a.fX[Cross<NDIM>::b(l, k)] + o.I, j));
+                Kv = zero_if(!in, [&] { return ldt<TILE>((const S*)a.fX[Cross<NDIM>::b(l, k)] + o.I, j); });
               } else {
                 if (in) {
                   T dxkj, rxkj;
@@ -581,8 +592,8 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
               K[sg] = Kv;
               Ke[sg] = Kv * ldt<TILE>(W(B0 + 1 + k), j);
             }
-            const T tC = zero_if(z1[l], over(K[1] - K[0], l) / T(2));
-            const T tCe = zero_if(z1[l], over(Ke[1] - Ke[0], l) / T(2));
+            const T tC = zero_if(z1[l], [&] { return over(K[1] - K[0], l) / T(2); });
+            const T tCe = zero_if(z1[l], [&] { return over(Ke[1] - Ke[0], l) / T(2); });
             acc[B0 + 1 + k] = acc[B0 + 1 + k] + T(-1) * tC * q2;
             acc[E] = acc[E] + T(-1) * tCe * q2;
           }
@@ -590,8 +601,8 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
           {
             const T qc = ldt<TILE>(q, c), qm = ldt<TILE>(q, c - sk), qp = ldt<TILE>(q, c + sk);
             const T BL = (qc + qm) / T(2), BR = (qp + qc) / T(2);
-            const T gL = zero_if(z1[k], over(qc - qm, k));
-            const T gR = zero_if(z1[k], over(qp - qc, k));
+            const T gL = zero_if(z1[k], [&] { return over(qc - qm, k); });
+            const T gR = zero_if(z1[k], [&] { return over(qp - qc, k); });
             const T tL = nl * gL, tR = nr * gR;
             acc[B0 + 1 + l] = acc[B0 + 1 + l] + over(T(1) * (tR - tL), k) * q2;
             acc[E] = acc[E] + over(T(1) * (tR * BR - tL * BL), k) * q2;
@@ -729,8 +740,12 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
 #pragma unroll
       for (int d = 0; d < NDIM; ++d) {
         const int s = st[d];
-        const T n4 = -(Bat(d, c + 2 * s) - T(8) * (Bat(d, c + s) - Bat(d, c - s)) - Bat(d, c - 2 * s));
-        const T gd = z4[d] ? T(0) : qdiv<FAST>(qdiv<FAST>(n4, dxv[d], rxv[d]), T(12), r12);
+        T gd = T(0);
+        if (SELECT || !z4[d]) {
+          const T n4 = -(Bat(d, c + 2 * s) - T(8) * (Bat(d, c + s) - Bat(d, c - s)) - Bat(d, c - 2 * s));
+          const T q4 = qdiv<FAST>(qdiv<FAST>(n4, dxv[d], rxv[d]), T(12), r12);
+          gd = z4[d] ? T(0) : q4;
+        }
         divb = divb + gd;
       }
       divb = q2 * divb;
@@ -1172,16 +1187,17 @@ void launch_update(const Stage2Args& a0, cudaStream_t st) {
     // they took 1.1 ms per step off the update for 0.43 ms of k_cross; in FP32 the
     // update falls from 521 us (inline, 32 registers) to 298 for 68 us of k_cross
     constexpr int P = OPT_PRE;
-    // a state with many cells out of range (a.quiet): the general form for all of it,
-    // in two launches at 5 and 4 blocks per SM.  At 128^3 from rest 6.6 ms per step so,
-    // 11 in the common kernel, whose registers leave its divides 16 warps per SM
+    // a state with many cells out of range (a.quiet), or a call whose every cell takes the
+    // general form: that form alone, in 3D without sources in two launches at 5 and 4
+    // blocks per SM.  A split sweep at 96^3 341 us so, 517 in the common kernel, whose
+    // registers leave its divides 16 warps per SM
     auto go = [&](auto o) {
       constexpr int O = P | decltype(o)::value;
-      if constexpr (NDIM == 3 && sizeof(S) == 8) {
-        if (a.quiet) {
-          const dim3 qblk(8, 8, 4);  // part B 729 us per launch so, 764 at 32x8x1
+      if constexpr (NDIM > 1 && sizeof(S) == 8) {
+        if (a.quiet || a.general) {
+          const dim3 qblk = NDIM == 3 ? dim3(8, 8, 4) : blk;  // part B 729 us per launch so, 764 at 32x8x1
           const dim3 qgrd((n0 + qblk.x - 1) / qblk.x, (n1 + qblk.y - 1) / qblk.y, (n2 + qblk.z - 1) / qblk.z);
-          if constexpr (O == P) {
+          if constexpr (O == P && NDIM == 3) {
             k_update<NDIM, NDIR, S, O | OPT_QUIET | OPT_PART_A><<<qgrd, qblk, 0, st>>>(a);
             k_update<NDIM, NDIR, S, O | OPT_QUIET | OPT_PART_B><<<qgrd, qblk, 0, st>>>(a);
           } else {
