@@ -32,11 +32,22 @@ using namespace sacgpu;
 
 namespace {
 constexpr double bigdouble = 1.0e99, smalldouble = 1.0e-99;
-// One cell in this many out of range (k_face) sends the FP64 3D update to the general
-// form's own kernels: at 128^3 its common kernel takes 0.67 ms per launch where no warp
-// meets such a cell and 2.2 where all do, those kernels 1.04 whatever the state, which is
-// even at 0.23 of the warps; the cells' stencils reach about twice as many
-constexpr long kQuietShare = 8;
+// The share of the FP64 update's warps with a stencil out of range (k_count_divides, in
+// percent) from which on every cell takes the general form, in kernels of its own.
+// Update plus k_face per launch, common kernels against those, in us:
+//   3D, 128^3             816 / 1081 at no such warp, 1106 / 1106 at 23 %, 1480 / 1123 at
+//                         63 %, 1835 / 1193 at 90 %
+//   3D with sources       886 / 1475 at none, 1829 / 1529 at 75 %: even near 50 %
+//   2D with sources       98 / 91 at 2 % of 512^2, 40 / 41 at 5 % of 200x160, 280 / 344 at
+//                         0.4 % of 1200x1000
+// In 2D without sources the common kernel has the general one's occupancy and wins at any
+// share (105 / 133 at 40 % of 512^2, 57.6 / 57.4 at 96 % of 200x160).
+constexpr long quiet_percent(int ndim, bool sources) {
+  return ndim == 3 ? (sources ? 50 : 23) : (ndim == 2 && sources ? 25 : 100);
+}
+// ... as counted in one stage of this many, whose k_face tests every field in the general
+// form's steps too (a launch of 4 to 13 us)
+constexpr unsigned kProbeStages = 16;
 }
 
 struct sac_ctx {
@@ -64,14 +75,15 @@ struct sac_ctx {
   double* drv = nullptr;
   double* stg = nullptr;  // FP64 staging block for FP32 upload/download
   double drvA = 0.0;
-  // 0 maxnu, 1 courant, 2..4 ctot, 5 cells out of range of the last step (32 bits); then
+  // 0 maxnu, 1 courant, 2 the warps counted by a probing stage (32 bits), 3..5 ctot; then
   // the FP64 stage's brick flags (one memset clears ctot and the flags)
   unsigned long long* red = nullptr;
-  // pinned words: maxnu and courant as getdt copied them, and the count above (FP64 3D)
-  // as of a recent step; the count chooses between kernels with the same results, so
-  // its age does not matter
+  // pinned words: maxnu and courant as getdt copied them, and the count above as of a
+  // recent step; the count chooses between kernels with the same results, so its age does
+  // not matter
   unsigned long long* h_red = nullptr;
   size_t nflags = 0;  // bytes of flags (0: FP32)
+  unsigned stages = 0;  // stages since sac_set_grid that could have probed
   unsigned long long* kp = nullptr;   // keeppositive's words (smallfix only), see k_keeppos_scan
   int it_now = 0;                     // the step number last passed to sac_getdt or sac_advect
   double* fixB = nullptr;
@@ -198,8 +210,6 @@ bool visc_on(const sac_ctx* c) {
   if (c->par.user == SAC_USR_NONE) return false;
   return std::fabs(c->par.nu) > smalldouble;
 }
-// the FP64 3D stage counts its cells out of range
-bool count_bad(const sac_ctx* c) { return c->g.ndim == 3 && c->prec == SAC_PREC_FP64; }
 bool grav_module(int u) {
   return u == SAC_USR_SLOG || u == SAC_USR_GRAVVISC || u == SAC_USR_STRAT || u == SAC_USR_TUBE;
 }
@@ -356,7 +366,7 @@ Stage2Args stage_args(sac_ctx* c, bool flux, double qdt, int dmin, int dmax, dou
   a.fst[1] = (g.n[0] + 7) / 8;
   a.fst[2] = a.fst[1] * ((g.n[1] + 7) / 8);
   a.drv = c->drv;
-  a.ctot = c->red + 2;
+  a.ctot = c->red + 3;
   a.maxnu = c->red;
   a.qdt = qdt;
   // sources inside centdiff4 carry qdt*(idimmax-idimmin+1)/ndim, src/vaccd.t:73-75;
@@ -383,8 +393,12 @@ Stage2Args stage_args(sac_ctx* c, bool flux, double qdt, int dmin, int dmax, dou
   if (a.res_on && (!(a.eta >= 0x1p-60 && a.eta <= 0x1p60) ||
                    !(std::fabs(a.qdt2) >= 0x1p-80 && std::fabs(a.qdt2) <= 0x1p60)))
     a.general = 1;
-  a.nbad = (unsigned*)(c->red + 5);
-  a.quiet = count_bad(c) && (long)*(volatile unsigned*)(c->h_red + 2) > g.ncell / kQuietShare ? 1 : 0;
+  a.nbad = (unsigned*)(c->red + 2);
+  const long quiet = quiet_percent(g.ndim, a.res_on || a.divb_on);
+  if (quiet < 100 && c->nflags && !a.general) {
+    a.quiet = 100L * *(volatile unsigned*)(c->h_red + 2) > quiet * count_warps(g) ? 1 : 0;
+    a.probe = c->stages++ % kProbeStages == 0 ? 1 : 0;
+  }
   a.driver = DRV_NONE;
   if (c->par.sourceunsplit && c->drv) {
     if (u == SAC_USR_SLOG && g.ndim == 3) {
@@ -422,9 +436,10 @@ sac_status advect1_t(sac_ctx* c, const std::string& method, double qdt, int dmin
                      const void* aux2) {
   const Geom& g = c->g;
   if (method == "cd4" || method == "source") {
-    CK(cudaMemsetAsync(c->red + 2, 0, 4 * sizeof(unsigned long long) + c->nflags, c->stream));
     const Stage2Args a =
         stage_args<S>(c, method == "cd4", qdt, dmin, dmax, qt, wct, base, out, mask, epi, aux1, aux2);
+    const int cleared = a.probe ? 4 : 3;  // the count where it is taken, ctot, the flags
+    CK(cudaMemsetAsync(c->red + 6 - cleared, 0, cleared * sizeof(unsigned long long) + c->nflags, c->stream));
     const bool visc = a.visc_on != 0;
     {
       Prof pr(c, SAC_K_PREP);
@@ -434,6 +449,11 @@ sac_status advect1_t(sac_ctx* c, const std::string& method, double qdt, int dmin
       Prof pr(c, SAC_K_NU);
       launch_nu<S>(a, c->stream);
       if (c->X) launch_cross<S>(a, c->stream);
+    }
+    if (a.probe) {
+      Prof pr(c, SAC_K_OTHER);
+      launch_count_divides(a, c->stream);
+      CK(cudaMemcpyAsync(c->h_red + 2, c->red + 2, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
     }
     {
       Prof pr(c, SAC_K_STAGE);
@@ -994,6 +1014,7 @@ sac_status sac_set_grid(sac_ctx* c, int ndim, int ndir, const int ixGhi[3], cons
   }
   CK(cudaMalloc(&c->red, 6 * sizeof(unsigned long long) + c->nflags));
   CK(cudaMemsetAsync(c->red, 0, 6 * sizeof(unsigned long long) + c->nflags, c->stream));
+  c->stages = 0;
   CK(cudaMallocHost(&c->h_red, 3 * sizeof(unsigned long long)));
   std::memset(c->h_red, 0, 3 * sizeof(unsigned long long));
   if (c->par.smallfix) {
@@ -1488,8 +1509,6 @@ sac_status sac_advect(sac_ctx* c, const char* method, const int* iws, int idimmi
     return fail(c, SAC_ERR_UNSUPPORTED, "typeadvance=" + ta);
   }
 #undef RUN
-  if (count_bad(c))
-    CK(cudaMemcpyAsync(c->h_red + 2, c->red + 5, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaGetLastError());
   return SAC_OK;
 }
@@ -1543,10 +1562,10 @@ sac_status sac_diag(sac_ctx* c, sac_diag_out* out) {
   });
   out->divb_l2 = std::sqrt(s2 / (double)n);
   out->divb_linf = mx;
-  unsigned long long bits[5];
+  unsigned long long bits[6];
   CK(cudaMemcpy(bits, c->red, sizeof(bits), cudaMemcpyDeviceToHost));
   std::memcpy(&out->maxviscoef, &bits[0], sizeof(double));
-  for (int d = 0; d < 3; ++d) std::memcpy(&out->ctot[d], &bits[2 + d], sizeof(double));
+  for (int d = 0; d < 3; ++d) std::memcpy(&out->ctot[d], &bits[3 + d], sizeof(double));
   out->nonfinite = nonfinite;
   if (c->kp) {
     unsigned long long kp[5];

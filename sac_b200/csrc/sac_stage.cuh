@@ -815,35 +815,21 @@ __global__ void __launch_bounds__(256, sizeof(S) == 8 ? SAC_FACE_MINB_F64 : SAC_
 #pragma unroll
   for (int d = 0; d < NDIM; ++d) cm[d] = 0.0;
   bool bad = false;
-  const bool sampled = blockIdx.x % 16 == 0;  // a.nbad counts one block in 16, which is enough for its use
   const int p0 = c % g.n[0], p1 = (c / g.n[0]) % g.n[1], p2 = c / (g.n[0] * g.n[1]);
   if (c < (int)g.ncell) {
     const bool mesh = do_ctot && p0 >= g.lo[0] && p0 <= g.hi[0] && p1 >= g.lo[1] && p1 <= g.hi[1] &&
                       p2 >= g.lo[2] && p2 <= g.hi[2];
-    bad = face_cell<NDIM, NDIR, S>(a, Offs{}, c, mesh, a.gamma, cm, sampled || !a.quiet);
+    bad = face_cell<NDIM, NDIR, S>(a, Offs{}, c, mesh, a.gamma, cm, !a.quiet || a.probe);
   }
   if constexpr (sizeof(S) == 8) {
-    // flag the bricks around each brick in which this warp has a cell out of range (a
-    // stencil reaches 3 cells): one lane per neighbour
+    // flag the bricks of this warp's cells out of range, one lane per run of cells in a
+    // brick (update warps look at the bricks that their stencils reach)
     const unsigned all = __ballot_sync(0xffffffffu, bad);
-    const int lane = threadIdx.x & 31;
-    if (all && !a.quiet) {  // the quiet form's kernels read no flags
-      const int brick = (p0 >> 3) + a.fst[1] * (p1 >> 3) + a.fst[2] * (p2 >> 3);
+    if (all) {
+      const int brick = (p0 >> 3) + a.fst[1] * (p1 >> 3) + a.fst[2] * (p2 >> 3), lane = threadIdx.x & 31;
       const int before = __shfl_up_sync(0xffffffffu, brick, 1);
-      const bool leads = bad && !(lane > 0 && ((all >> (lane - 1)) & 1u) && before == brick);
-      for (unsigned m = __ballot_sync(0xffffffffu, leads); m; m &= m - 1) {
-        const int src = __ffs(m) - 1;
-        const int b0 = (__shfl_sync(0xffffffffu, p0, src) >> 3) + lane % 3 - 1;
-        const int b1 = (__shfl_sync(0xffffffffu, p1, src) >> 3) + (lane / 3) % 3 - 1;
-        const int b2 = (__shfl_sync(0xffffffffu, p2, src) >> 3) + lane / 9 - 1;
-        if (lane < 27 && b0 >= 0 && b0 <= (g.n[0] - 1) >> 3 && b1 >= 0 && b1 <= (g.n[1] - 1) >> 3 && b2 >= 0 &&
-            b2 <= (g.n[2] - 1) >> 3) {
-          unsigned char* f = a.flags + b0 + a.fst[1] * b1 + a.fst[2] * b2;
-          if (!__ldcg(f)) *f = 1;  // most are set: reads of a hot sector do not queue as writes do
-        }
-      }
+      if (bad && !(lane > 0 && ((all >> (lane - 1)) & 1u) && before == brick)) a.flags[brick] = 1;
     }
-    if (NDIM == 3 && all && sampled && lane == 0) atomicAdd(a.nbad, 16u * (unsigned)__popc(all));
   }
   if (do_ctot) {
 #pragma unroll
@@ -869,19 +855,45 @@ __global__ void __launch_bounds__(256, sizeof(S) == 8 ? SAC_NU_MINB_F64 : SAC_NU
   nu_cell<NDIM, NDIR, S>(a, g, Offs{}, c, p, a.ctot);
 }
 
-// Whether the cells of this warp take the general form (FAST = false): the launch
-// does, or in FP64 a brick that one of them lies in is flagged or setnu's c_tot is out
-// of range (in: this thread has a mesh cell, at pos)
-template <int NDIM, typename S>
-__device__ __forceinline__ bool takes_divide(const Stage2Args& a, bool in, const int pos[3]) {
-  bool slow = a.general || a.quiet;
-  if constexpr (sizeof(S) != 8) return slow;
+// Whether a field within 3 cells (the stencils' reach) of this warp's 32 cells along x1
+// is out of range, or setnu's c_tot (FP64): the bricks that the row and its surroundings
+// touch, one lane each.  All lanes of the warp take part; pos is this lane's cell.
+template <int NDIM>
+__device__ __forceinline__ bool row_out_of_range(const Stage2Args& a, const int pos[3]) {
+  const Geom& g = a.g;
+  const int lane = threadIdx.x & 31, x0 = pos[0] - lane;
+  const int i = lane % 6, j = lane / 6 % 2, k = lane / 12;  // 35 + 3 cells touch 6 bricks, 7 cells 2
+  const int b0 = max((x0 - 3) >> 3, 0) + i;
+  bool bad = false;
+  if (b0 <= min(x0 + 34, g.n[0] - 1) >> 3 && j < (NDIM > 1 ? 2 : 1) && k < (NDIM > 2 ? 2 : 1)) {
+    const int b1 = NDIM > 1 ? min(max(pos[1] + (j ? 3 : -3), 0), g.n[1] - 1) >> 3 : 0;
+    const int b2 = NDIM > 2 ? min(max(pos[2] + (k ? 3 : -3), 0), g.n[2] - 1) >> 3 : 0;
+    bad = __ldg(a.flags + b0 + a.fst[1] * b1 + a.fst[2] * b2) != 0;
+  }
   if (a.visc_on) {
 #pragma unroll
-    for (int d = 0; d < NDIM; ++d) slow = slow || ctot_out_of_range(a.ctot[d]);
+    for (int d = 0; d < NDIM; ++d) bad = bad || ctot_out_of_range(a.ctot[d]);
   }
-  if (in) slow = slow || __ldg(a.flags + (pos[0] >> 3) + a.fst[1] * (pos[1] >> 3) + a.fst[2] * (pos[2] >> 3)) != 0;
-  return __any_sync(0xffffffffu, slow);
+  return __any_sync(0xffffffffu, bad);
+}
+
+// Whether the cells of this warp take the general form (FAST = false)
+template <int NDIM, typename S>
+__device__ __forceinline__ bool takes_divide(const Stage2Args& a, const int pos[3]) {
+  if (a.general || a.quiet) return true;
+  if constexpr (sizeof(S) == 8) return row_out_of_range<NDIM>(a, pos);
+  return false;
+}
+
+// the number of warps of the update's common kernel that take the general form, for the
+// choice of the next steps' kernels (a.quiet); blocks of 32 x 8 cells, as that kernel's
+template <int NDIM>
+__global__ void __launch_bounds__(256) k_count_divides(const Stage2Args a) {
+  const int pos[3] = {a.g.lo[0] + (int)(blockIdx.x * blockDim.x + threadIdx.x),
+                      a.g.lo[1] + (int)(blockIdx.y * blockDim.y + threadIdx.y), a.g.lo[2] + (int)blockIdx.z};
+  const bool in = pos[1] <= a.g.hi[1];  // (a warp's rows begin inside along x1)
+  const int n = __syncthreads_count(row_out_of_range<NDIM>(a, pos) && in && (threadIdx.x & 31) == 0);
+  if (threadIdx.x == 0 && threadIdx.y == 0 && n) atomicAdd(a.nbad, (unsigned)n);
 }
 
 // k_cross body at the mesh cell pos: for every l != k the centred half-sums of
@@ -938,7 +950,7 @@ __global__ void __launch_bounds__(256, SAC_CROSS_MINB) k_cross(const Stage2Args 
   pos[1] = g.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
   pos[2] = g.lo[2] + blockIdx.z * blockDim.z + threadIdx.z;
   const bool in = pos[0] <= g.hi[0] && pos[1] <= g.hi[1] && pos[2] <= g.hi[2];
-  const bool slow = takes_divide<NDIM, S>(a, in, pos);
+  const bool slow = takes_divide<NDIM, S>(a, pos);
   if (!in) return;
   if (slow)
     cross_cell<NDIM, NDIR, S, false>(a, g, Offs{}, pos);
@@ -974,7 +986,7 @@ __global__ void __launch_bounds__(256, update_minb<S, NDIM, OPT>())
     if (in) update_cell<NDIM, NDIR, S, OPT, false>(a, g, Offs{}, pos, a.qdt, a.qdt2, a.tdep, a.drvA, numax);
     if constexpr ((OPT & OPT_PART_A) != 0) return;
   } else {
-    const bool slow = takes_divide<NDIM, S>(a, in, pos);
+    const bool slow = takes_divide<NDIM, S>(a, pos);
     if (in) {
       if (slow)
         update_cell<NDIM, NDIR, S, OPT, false>(a, g, Offs{}, pos, a.qdt, a.qdt2, a.tdep, a.drvA, numax);
@@ -1189,8 +1201,9 @@ void launch_update(const Stage2Args& a0, cudaStream_t st) {
     constexpr int P = OPT_PRE;
     // a state with many cells out of range (a.quiet), or a call whose every cell takes the
     // general form: that form alone, in 3D without sources in two launches at 5 and 4
-    // blocks per SM.  A split sweep at 96^3 341 us so, 517 in the common kernel, whose
-    // registers leave its divides 16 warps per SM
+    // blocks per SM.  At 128^3 from rest (90 % of the warps) 1.02 ms per launch so, 1.62 in
+    // the common kernel, whose registers leave its divides 16 warps per SM; a split sweep
+    // at 96^3 341 us so, 517 there
     auto go = [&](auto o) {
       constexpr int O = P | decltype(o)::value;
       if constexpr (NDIM > 1 && sizeof(S) == 8) {

@@ -55,16 +55,17 @@ struct Stage2Args {
   const void* xr[3];
   int axis_tab;
   // brick flags of the FP64 single grid (k_face): a brick of 8 cells per dimension is
-  // set where a cell within one brick of it holds a field out of range, and its cells
-  // then take the divides; brick strides fst
+  // set where one of its cells holds a field out of range, and the cells whose stencils
+  // reach it then take the divides; brick strides fst
   unsigned char* flags;
   int fst[3];
   const double* dx[3];  // cell widths per cell (the batch's getdt_courant)
-  unsigned* nbad;       // count of the cells with a field out of range (FP64, 3D)
   // every cell takes the update's general form: a split sweep (dmin..dmax), a partial
   // variable list (iwmask), or widths, eta or the step out of range
   int general;
-  int quiet;            // many cells out of range: the general form's own kernels (FP64, 3D)
+  int quiet;       // so does every cell of a state with many out of range (FP64)
+  int probe;       // this stage counts the warps that take the divides, into nbad
+  unsigned* nbad;
   const double* drv; // driver profiles [2][N] or nullptr
   const unsigned long long* ctot;
   unsigned long long* maxnu;
@@ -127,6 +128,12 @@ template <typename S>
 void launch_update(const Stage2Args& a, cudaStream_t st);
 template <typename S>
 void launch_cross(const Stage2Args& a, cudaStream_t st);
+// a stage with a.probe: the warps of k_update's common kernel that take the divides
+// (FP64, 2D and 3D), counted into a.nbad; there are count_warps of them
+void launch_count_divides(const Stage2Args& a, cudaStream_t st);
+inline long count_warps(const Geom& g) {
+  return (long)((g.hi[0] - g.lo[0] + 32) / 32) * (g.hi[1] - g.lo[1] + 1) * (g.hi[2] - g.lo[2] + 1);
+}
 
 // a whole RK4 step of a small 1D grid in one launch (sac_step1d.cuh): the four stages'
 // arguments and boundary fills; the largest shared memory such a grid may take

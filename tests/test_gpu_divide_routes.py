@@ -11,6 +11,7 @@ from oracle.oracle import Oracle
 from sac_b200 import abi, problems
 
 import _util
+from test_gpu_batch import _batch_of, _ot_problems
 
 pytestmark = pytest.mark.gpu
 
@@ -57,9 +58,72 @@ CELLS = {2: [(14, 22), (29, 17), (0, 0), (42, 37)], 3: [(14, 22, 6), (29, 25, 17
 
 
 @pytest.mark.parametrize("sources", [False, True])
+@pytest.mark.parametrize("nx,ndir", [((43, 38), 2), ((43, 38), 3), ((43, 38, 35), 3)])
+def test_single_cells_out_of_range(nx, ndir, sources):
+    """Six, six and five bricks per side: a cell's divides and its neighbours' fast form,
+    each cell by itself and all together."""
+    for cells in [[q] for q in CELLS[len(nx)]] + [CELLS[len(nx)]]:
+        P = _problem(nx, ndir, sources)
+        _tiny(P, cells)
+        route = _steps_equal(P, 2)
+        # away from the periodic ends a cell reaches 14 x 14 of the 38 x 35 rows
+        if len(nx) == 3 and cells in [[q] for q in CELLS[3][:3]]:
+            assert route == [0, 0]
+
+
+@pytest.mark.parametrize("typ", ["periodic", "cont"])
+@pytest.mark.parametrize("sources", ["none", "powell", "res", "all"])
+@pytest.mark.parametrize("nx,ndir", [((43, 38), 2), ((43, 38), 3), ((43, 38, 35), 3)])
+def test_many_cells_out_of_range(nx, ndir, sources, typ):
+    """A state out of range in all but a corner: the first stage counts its warps and the
+    steps after it run the general form's own kernels (not in 2D without sources)."""
+    P = _problem(nx, ndir, False, typ)
+    if sources in ("powell", "all"):
+        P.params.divbfix = 1
+    if sources in ("res", "all"):
+        P.params.eta = 0.01
+    v = problems.var_index(ndir)
+    corner = tuple(slice(0, 9) for _ in nx)
+    keep = P.w[corner].copy()
+    P.w[..., 1:1 + ndir] *= 1e-70
+    P.w[..., v["b0"] + 1:v["b0"] + 1 + ndir] *= 1e-70
+    P.w[..., v["bg0"] + 1:] *= 1e-75
+    P.params.grav[:] = [0.0, 0.0, 0.0]
+    P.w[corner] = keep
+    route = _steps_equal(P, 3)
+    assert route[1:] == ([1, 1] if len(nx) == 3 or sources != "none" else [0, 0])
+
+
+@pytest.mark.parametrize("sources", [False, True])
 @pytest.mark.parametrize("nx,ndir", [((43, 38), 2), ((43, 38, 35), 3)])
 def test_split_sweeps_and_variable_lists(nx, ndir, sources):
     for kw in (dict(idimmin=2, idimmax=2), dict(iws=[1, 2, ndir + 2])):
         P = _problem(nx, ndir, sources)
         _tiny(P, CELLS[len(nx)])
         assert _steps_equal(P, 2, **kw) == [1, 1]
+
+
+@pytest.mark.parametrize("nx,cells", [(60, [(14,), (59,)]), (125, [(0,), (62,)]), (800, [(99,), (100,), (500,)]),
+                                      (333, [((0, 333),)])])
+def test_1d_step_with_cells_out_of_range(nx, cells):
+    """The one-launch 1D step, cells at the ends of the clusters' segments among them."""
+    P = _problem((nx,), 2, False)
+    _tiny(P, cells)
+    _steps_equal(P, 3)
+
+
+@pytest.mark.parametrize("shape", [0, 1])
+def test_fused_batch_stage_with_cells_out_of_range(shape):
+    """A tile's one vote for its divides: the fused stage and the three passes, whose update
+    divides everywhere, agree bit for bit."""
+    Ps = _ot_problems([(40, 24), (64, 72), (70, 64)], [0.6, 2.5, 9.0])
+    _tiny(Ps[0], [(31, 7)])
+    _tiny(Ps[1], [(14, 22), (0, 0), (63, 71)])
+    _tiny(Ps[2], [((0, 70), (0, 20))])
+    a, f = (_batch_of(Ps, Ps[0].params) for _ in range(2))
+    a.set_stage(False)
+    f.set_stage(True, shape)
+    for _ in range(3):
+        a.advance(1)
+        f.advance(1)
+        np.testing.assert_array_equal(f.download(), a.download())
