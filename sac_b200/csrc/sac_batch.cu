@@ -311,7 +311,7 @@ Stage2Args stage_base(sac_batch* b) {
   a.F = b->F;
   a.R = b->R;
   for (int d = 0; d < b->ndim; ++d) a.dx[d] = b->dx + (size_t)d * b->totX;
-  for (int d = 0; d < b->ndim; ++d) a.xr[d] = (const char*)b->xr + 2 * b->es * b->xr_off[d];
+  for (int d = 0; d < b->ndim; ++d) a.xr[d] = b->xr ? (const char*)b->xr + 2 * b->es * b->xr_off[d] : nullptr;
   a.axis_tab = b->axis_tab;
   a.general = b->widths_ok ? 0 : 1;
   a.gamma = b->par.gamma;
@@ -804,28 +804,29 @@ sac_status sac_batch_set_grid(sac_batch* b, const double* x) {
     BK(cudaMemset(p, 0, es * b->np * b->totP));  // scratch stages of finished instances stay finite
   }
   BK(cudaMalloc(&b->BG, sizeof(double) * (b->nw - b->np) * b->totP));
-  // the widths' table, per index along each dimension where every instance allows it
+  // the widths' table, where every instance's vary along their own dimension alone
   b->axis_tab = tab ? 1 : 0;
-  b->widths_ok = true;
   std::vector<double> xr64;
   std::vector<float> xr32;
-  for (int d = 0; d < ndim; ++d) {
-    const long first = (long)(b->prec == SAC_PREC_FP32 ? xr32.size() : xr64.size()) / 2;
-    b->xr_off[d] = first;
-    for (int i = 0; i < b->ninst; ++i) {
-      const Geom& g = b->h_inst[i].g;
-      const double* q = hdx.data() + (size_t)d * b->totX + b->h_inst[i].o.X;
-      b->h_inst[i].o.A[d] = (int)((long)(b->prec == SAC_PREC_FP32 ? xr32.size() : xr64.size()) / 2 - first);
-      if (b->prec == SAC_PREC_FP32)
-        append_width_pairs(xr32, g.n, g.lo, g.hi, ndim, g.ncell, q, d, tab);
-      else
-        b->widths_ok &= append_width_pairs(xr64, g.n, g.lo, g.hi, ndim, g.ncell, q, d, tab);
+  if (tab)
+    for (int d = 0; d < ndim; ++d) {
+      b->xr_off[d] = (long)(xr64.size() + xr32.size()) / 2;
+      for (int i = 0; i < b->ninst; ++i) {
+        const Geom& g = b->h_inst[i].g;
+        const double* q = hdx.data() + (size_t)d * b->totX + b->h_inst[i].o.X;
+        b->h_inst[i].o.A[d] = (int)((long)(xr64.size() + xr32.size()) / 2 - b->xr_off[d]);
+        if (b->prec == SAC_PREC_FP32) append_width_pairs(xr32, g.n, g.lo, g.hi, ndim, q, d);
+        else append_width_pairs(xr64, g.n, g.lo, g.hi, ndim, q, d);
+      }
     }
-  }
+  b->widths_ok = b->prec == SAC_PREC_FP32 || (tab ? widths_in_range(xr64.data(), (long)xr64.size(), 2)
+                                                  : widths_in_range(hdx.data(), (long)hdx.size(), 1));
   const size_t xr_bytes = xr64.size() * sizeof(double) + xr32.size() * sizeof(float);
-  BK(cudaMalloc(&b->xr, xr_bytes));
-  BK(cudaMemcpy(b->xr, xr64.empty() ? (const void*)xr32.data() : (const void*)xr64.data(), xr_bytes,
-                cudaMemcpyHostToDevice));
+  if (xr_bytes) {
+    BK(cudaMalloc(&b->xr, xr_bytes));
+    BK(cudaMemcpy(b->xr, xr64.empty() ? (const void*)xr32.data() : (const void*)xr64.data(), xr_bytes,
+                  cudaMemcpyHostToDevice));
+  }
   BK(cudaMalloc(&b->dx, sizeof(double) * ndim * b->totX));
   BK(cudaMemcpy(b->dx, hdx.data(), sizeof(double) * hdx.size(), cudaMemcpyHostToDevice));
   if (gauss) {
@@ -868,6 +869,16 @@ sac_status sac_batch_set_grid(sac_batch* b, const double* x) {
   }
   if ((st = upload_vec(b, &b->d_dyn, dyn)) != SAC_OK) return st;
   if ((st = build_lists(b)) != SAC_OK) return st;
+  if (!tab) {  // after everything else, see width_pairs_per_cell
+    for (int d = 0; d < ndim; ++d) b->xr_off[d] = d * b->totX;
+    if (b->prec == SAC_PREC_FP32) {
+      BK(width_pairs_per_cell<float>(b->dx, ndim * b->totX, &b->xr, b->stream));
+    } else if (b->widths_ok) {
+      BK(width_pairs_per_cell<double>(b->dx, ndim * b->totX, &b->xr, b->stream));
+      b->widths_ok = b->xr != nullptr;
+    }
+    BK(cudaStreamSynchronize(b->stream));
+  }
   b->grid_set = true;
   return SAC_OK;
 }

@@ -66,22 +66,22 @@ struct sac_ctx {
   void* F = nullptr;
   void* R = nullptr;
   void* X = nullptr;  // cross-derivative half-sums (k_cross), allocated with hyperdiffusion
-  double* x = nullptr;
   double* dx = nullptr;
   void* xr = nullptr;  // cell widths with their reciprocals (Stage2Args::xr)
   long xr_off[3] = {0, 0, 0};  // pairs before dimension d's
   int axis_tab = 0;
-  bool widths_ok = true;  // the widths are in qdiv's range
+  bool widths_ok = true;  // the widths are in qdiv's range, with their reciprocals in xr
   double* drv = nullptr;
   double* stg = nullptr;  // FP64 staging block for FP32 upload/download
   double drvA = 0.0;
   // 0 maxnu, 1 courant, 2 the warps counted by a probing stage (32 bits), 3..5 ctot; then
   // the FP64 stage's brick flags (one memset clears ctot and the flags)
   unsigned long long* red = nullptr;
-  // pinned words: maxnu and courant as getdt copied them, and the count above as of a
-  // recent step; the count chooses between kernels with the same results, so its age does
-  // not matter
-  unsigned long long* h_red = nullptr;
+  // maxnu and courant as getdt copied them, and the count above, which getdt brings along
+  // where a stage took it; it chooses between kernels with the same results, so its age
+  // does not matter
+  unsigned long long h_red[3] = {0, 0, 0};
+  bool count_taken = false;
   size_t nflags = 0;  // bytes of flags (0: FP32)
   unsigned stages = 0;  // stages since sac_set_grid that could have probed
   unsigned long long* kp = nullptr;   // keeppositive's words (smallfix only), see k_keeppos_scan
@@ -217,15 +217,13 @@ bool grav_module(int u) {
 void release(sac_ctx* c) {
   for (auto& p : c->P)
     if (p) cudaFree(p), p = nullptr;
-  for (void* p : {(void*)c->BG, c->D, c->F, c->R, c->X, (void*)c->x, (void*)c->dx, c->xr, (void*)c->drv,
+  for (void* p : {(void*)c->BG, c->D, c->F, c->R, c->X, (void*)c->dx, c->xr, (void*)c->drv,
                   (void*)c->stg, (void*)c->red, (void*)c->kp, (void*)c->fixB, (void*)c->d_type,
                   (void*)c->d_fixed})
     if (p) cudaFree(p);
-  c->BG = c->x = c->dx = c->drv = c->stg = c->fixB = nullptr;
+  c->BG = c->dx = c->drv = c->stg = c->fixB = nullptr;
   c->D = c->F = c->R = c->X = c->xr = nullptr;
   c->red = c->kp = nullptr;
-  if (c->h_red) cudaFreeHost(c->h_red);
-  c->h_red = nullptr;
   c->d_type = nullptr;
   c->d_fixed = nullptr;
 }
@@ -359,7 +357,8 @@ Stage2Args stage_args(sac_ctx* c, bool flux, double qdt, int dmin, int dmax, dou
   a.R = c->R;
   a.X = c->X;
   const size_t pair = 2 * c->es;
-  for (int d = 0; d < g.ndim; ++d) a.xr[d] = (const char*)c->xr + pair * c->xr_off[d];
+  for (int d = 0; d < g.ndim; ++d) a.xr[d] = c->xr ? (const char*)c->xr + pair * c->xr_off[d] : nullptr;
+  for (int d = 0; d < g.ndim; ++d) a.dx[d] = c->dx + (size_t)d * g.ncell;
   a.axis_tab = c->axis_tab;
   a.flags = (unsigned char*)(c->red + 6);
   a.fst[0] = 1;
@@ -396,7 +395,7 @@ Stage2Args stage_args(sac_ctx* c, bool flux, double qdt, int dmin, int dmax, dou
   a.nbad = (unsigned*)(c->red + 2);
   const long quiet = quiet_percent(g.ndim, a.res_on || a.divb_on);
   if (quiet < 100 && c->nflags && !a.general) {
-    a.quiet = 100L * *(volatile unsigned*)(c->h_red + 2) > quiet * count_warps(g) ? 1 : 0;
+    a.quiet = 100L * (long)(unsigned)c->h_red[2] > quiet * count_warps(g) ? 1 : 0;
     a.probe = c->stages++ % kProbeStages == 0 ? 1 : 0;
   }
   a.driver = DRV_NONE;
@@ -453,7 +452,7 @@ sac_status advect1_t(sac_ctx* c, const std::string& method, double qdt, int dmin
     if (a.probe) {
       Prof pr(c, SAC_K_OTHER);
       launch_count_divides(a, c->stream);
-      CK(cudaMemcpyAsync(c->h_red + 2, c->red + 2, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+      c->count_taken = true;
     }
     {
       Prof pr(c, SAC_K_STAGE);
@@ -946,7 +945,6 @@ sac_status sac_set_grid(sac_ctx* c, int ndim, int ndir, const int ixGhi[3], cons
         }
     c->mindx2[d] = m2;
   }
-  c->h_dx = hdx;
   // cell offsets inside one block of np (or ndir+3) fields are 32-bit
   if ((long)std::max(g.np, ndir + 3) * N > 2147483647L)
     return fail(c, SAC_ERR_UNSUPPORTED, "grid too large for 32-bit in-block indexing");
@@ -985,26 +983,26 @@ sac_status sac_set_grid(sac_ctx* c, int ndim, int ndir, const int ixGhi[3], cons
   CK(cudaMalloc(&c->R, c->es * (size_t)nr_pairs(ndim) * N));
   if (visc_on(c) && ndim > 1)  // the update reads them (k_cross)
     CK(cudaMalloc(&c->X, c->es * (size_t)n_cross(ndim) * N));
-  CK(cudaMalloc(&c->x, sizeof(double) * ndim * N));
   CK(cudaMalloc(&c->dx, sizeof(double) * ndim * N));
-  // the widths' table: per index along each dimension where they allow it
+  // the widths' table, where they vary along their own dimension alone
   c->axis_tab = widths_on_axes(g.n, g.lo, g.hi, ndim, N, hdx.data()) ? 1 : 0;
-  c->widths_ok = true;
   std::vector<double> xr64;
   std::vector<float> xr32;
-  for (int d = 0; d < ndim; ++d) {
-    if (c->prec == SAC_PREC_FP32) {
-      c->xr_off[d] = (long)xr32.size() / 2;
-      append_width_pairs(xr32, g.n, g.lo, g.hi, ndim, N, hdx.data() + (size_t)d * N, d, c->axis_tab != 0);
-    } else {
-      c->xr_off[d] = (long)xr64.size() / 2;
-      c->widths_ok &= append_width_pairs(xr64, g.n, g.lo, g.hi, ndim, N, hdx.data() + (size_t)d * N, d, c->axis_tab != 0);
+  if (c->axis_tab)
+    for (int d = 0; d < ndim; ++d) {
+      const double* q = hdx.data() + (size_t)d * N;
+      c->xr_off[d] = (long)(xr64.size() + xr32.size()) / 2;
+      if (c->prec == SAC_PREC_FP32) append_width_pairs(xr32, g.n, g.lo, g.hi, ndim, q, d);
+      else append_width_pairs(xr64, g.n, g.lo, g.hi, ndim, q, d);
     }
-  }
+  c->widths_ok = c->prec == SAC_PREC_FP32 || (c->axis_tab ? widths_in_range(xr64.data(), (long)xr64.size(), 2)
+                                                          : widths_in_range(hdx.data(), (long)hdx.size(), 1));
   const size_t xr_bytes = xr64.size() * sizeof(double) + xr32.size() * sizeof(float);
-  CK(cudaMalloc(&c->xr, xr_bytes));
-  CK(cudaMemcpyAsync(c->xr, xr64.empty() ? (const void*)xr32.data() : (const void*)xr64.data(), xr_bytes,
-                     cudaMemcpyHostToDevice, c->stream));
+  if (xr_bytes) {
+    CK(cudaMalloc(&c->xr, xr_bytes));
+    CK(cudaMemcpyAsync(c->xr, xr64.empty() ? (const void*)xr32.data() : (const void*)xr64.data(), xr_bytes,
+                       cudaMemcpyHostToDevice, c->stream));
+  }
   if (!hdrv.empty()) CK(cudaMalloc(&c->drv, sizeof(double) * 2 * N));
   if (c->prec == SAC_PREC_FP32) CK(cudaMalloc(&c->stg, sizeof(double) * g.np * N));
   c->nflags = 0;
@@ -1015,19 +1013,28 @@ sac_status sac_set_grid(sac_ctx* c, int ndim, int ndir, const int ixGhi[3], cons
   CK(cudaMalloc(&c->red, 6 * sizeof(unsigned long long) + c->nflags));
   CK(cudaMemsetAsync(c->red, 0, 6 * sizeof(unsigned long long) + c->nflags, c->stream));
   c->stages = 0;
-  CK(cudaMallocHost(&c->h_red, 3 * sizeof(unsigned long long)));
-  std::memset(c->h_red, 0, 3 * sizeof(unsigned long long));
+  std::memset(c->h_red, 0, sizeof(c->h_red));
+  c->count_taken = false;
   if (c->par.smallfix) {
     static const unsigned long long kp0[5] = {0, ~0ull, 0, 0, ~0ull};
     CK(cudaMalloc(&c->kp, sizeof(kp0)));
     CK(cudaMemcpyAsync(c->kp, kp0, sizeof(kp0), cudaMemcpyHostToDevice, c->stream));
   }
   CK(cudaMemsetAsync(c->R, 0, c->es * (size_t)nr_pairs(ndim) * N, c->stream));
-  CK(cudaMemcpyAsync(c->x, hx.data(), sizeof(double) * ndim * N, cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(c->dx, hdx.data(), sizeof(double) * ndim * N, cudaMemcpyHostToDevice, c->stream));
   if (!hdrv.empty())
     CK(cudaMemcpyAsync(c->drv, hdrv.data(), sizeof(double) * 2 * N, cudaMemcpyHostToDevice, c->stream));
+  if (!c->axis_tab) {  // after everything else, see width_pairs_per_cell
+    for (int d = 0; d < ndim; ++d) c->xr_off[d] = d * N;
+    if (c->prec == SAC_PREC_FP32) {
+      CK(width_pairs_per_cell<float>(c->dx, ndim * N, &c->xr, c->stream));
+    } else if (c->widths_ok) {
+      CK(width_pairs_per_cell<double>(c->dx, ndim * N, &c->xr, c->stream));
+      c->widths_ok = c->xr != nullptr;
+    }
+  }
   CK(cudaStreamSynchronize(c->stream));
+  c->h_dx = std::move(hdx);
   c->grid_set = true;
   c->bc_set = false;
   c->state_set = false;
@@ -1339,11 +1346,12 @@ static sac_status getdt_impl(sac_ctx* c, double* dt, int it, bool static_scratch
       else
         launch(0.0);
       }
-      // both maxima in one copy and one wait; courant starts the next call at zero
-      CK(cudaMemcpyAsync(c->h_red, c->red, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
+      // both maxima and the count in one copy and one wait; courant starts the next call at zero
+      CK(cudaMemcpyAsync(c->h_red, c->red, sizeof(c->h_red), cudaMemcpyDeviceToHost, c->stream));
       CK(cudaMemsetAsync(c->red + 1, 0, sizeof(unsigned long long), c->stream));
       CK(cudaStreamSynchronize(c->stream));
       have_maxnu = true;
+      c->count_taken = false;
       double courantmax;
       std::memcpy(&courantmax, c->h_red + 1, sizeof(double));
       if (!(courantmax == courantmax) || std::isinf(courantmax))
@@ -1382,6 +1390,11 @@ static sac_status getdt_impl(sac_ctx* c, double* dt, int it, bool static_scratch
     }
     if (c->par.dtcantgrow && it > c->itmin) d = std::min(d, c->dtold);
     c->dtold = d;
+  }
+  if (c->count_taken) {  // no copy above brought it
+    CK(cudaMemcpyAsync(c->h_red + 2, c->red + 2, sizeof(c->h_red[2]), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    c->count_taken = false;
   }
   *dt = d;
   return SAC_OK;

@@ -123,31 +123,29 @@ inline bool widths_on_axes(const int n[3], const int lo[3], const int hi[3], int
   return true;
 }
 
-// (dx, 1/dx) pairs of S, appended to out: the rows above (tab), or one per cell.
-// False where a width is outside the range of the stage's divisions through its
-// reciprocal (qdiv, out_of_range).
+// (dx, 1/dx) pairs of S of the rows above, appended to out
 template <typename S>
-inline bool append_width_pairs(std::vector<S>& out, const int n[3], const int lo[3], const int hi[3], int ndim,
-                               long ncell, const double* q, int d, bool tab) {
+inline void append_width_pairs(std::vector<S>& out, const int n[3], const int lo[3], const int hi[3], int ndim,
+                               const double* q, int d) {
   const long st[3] = {1, n[0], (long)n[0] * n[1]};
-  bool in_range = true;
-  auto put = [&](double v) {
-    in_range = in_range && v >= 0x1p-40 && v <= 0x1p40;
-    out.push_back((S)v);
-    out.push_back((S)(1.0 / v));
-  };
-  if (!tab) {
-    out.reserve(out.size() + 2 * ncell);
-    for (long i = 0; i < ncell; ++i) put(q[i]);
-    return in_range;
-  }
   for (int r = 0; r < 2 * ndim - 1; ++r) {
     int a[3], b[3];
     width_row(lo, hi, d, r, a, b);
     const long first = a[0] + st[1] * a[1] + st[2] * a[2] - st[d] * a[d];
-    for (long i = 0; i < n[d]; ++i) put(q[first + st[d] * i]);
+    for (long i = 0; i < n[d]; ++i) {
+      const double v = q[first + st[d] * i];
+      out.push_back((S)v);
+      out.push_back((S)(1.0 / v));
+    }
   }
-  return in_range;
+}
+
+// whether the widths (every step-th value) are in the range of the stage's divisions
+// through their reciprocals (qdiv, out_of_range)
+inline bool widths_in_range(const double* v, long n, int step) {
+  bool ok = true;
+  for (long i = 0; i < n; i += step) ok &= v[i] >= 0x1p-40 && v[i] <= 0x1p40;
+  return ok;
 }
 
 // Spatial profiles of the Gaussian velocity drivers on the full grid, two

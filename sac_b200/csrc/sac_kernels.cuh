@@ -153,6 +153,30 @@ __device__ __forceinline__ bool out_of_range(double x) {
   return (hi - kRangeLo) >= (kRangeHi - kRangeLo) && x != 0.0;
 }
 
+// (dx, 1/dx) pairs of S from the widths of n cells
+template <typename S>
+__global__ void k_width_pairs(const double* __restrict__ dx, S* __restrict__ out, long n) {
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+    out[2 * i] = (S)dx[i];
+    out[2 * i + 1] = (S)(1.0 / dx[i]);
+  }
+}
+
+// The table of pairs per cell of a grid whose widths do not vary along their own dimension
+// alone (n widths on the device).  In FP64, where the general form does without it, it is
+// made only where twice its size is free; nullptr in *out otherwise.
+template <typename S>
+inline cudaError_t width_pairs_per_cell(const double* dx, long n, void** out, cudaStream_t st) {
+  const size_t bytes = 2 * sizeof(S) * (size_t)n;
+  size_t avail = 0, total = 0;
+  cudaError_t e = cudaMemGetInfo(&avail, &total);
+  if (e != cudaSuccess || (sizeof(S) == 8 && avail < 2 * bytes)) return e;
+  e = cudaMalloc(out, bytes);
+  if (e != cudaSuccess) return e;
+  k_width_pairs<S><<<592, 256, 0, st>>>(dx, (S*)*out, n);
+  return cudaGetLastError();
+}
+
 // setnu's c_tot (the bits of a maximum of wave speeds) outside {0} and [2^-100, 2^200]
 __device__ __forceinline__ bool ctot_out_of_range(unsigned long long bits) {
   return bits != 0ull && (bits < ((1023ull - 100) << 52) || bits > ((1023ull + 200) << 52));

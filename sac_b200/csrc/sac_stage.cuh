@@ -48,10 +48,17 @@ __device__ __forceinline__ S ldt(const S* p, I i) {
 // ---------------------------------------------------------------------------
 // per-cell bodies (one grid, located by the offsets o)
 // ---------------------------------------------------------------------------
-// (width, reciprocal) of dimension d: from the axis table at index pd along d, or
-// per cell at cc
-template <typename S>
+// (width, reciprocal) of dimension d: from the axis table at index pd along d where the
+// grid has one, else from the table per cell at cc.  An FP64 grid may do without either
+// (a.xr), its cells all in the general form, which needs no reciprocal.
+template <bool FAST, typename S>
 __device__ __forceinline__ void width_at(const Stage2Args& a, const Offs& o, int d, int pd, long cc, S& dx, S& rx) {
+  if constexpr (!FAST && sizeof(S) == 8) {
+    if (!a.xr[d]) {
+      dx = __ldg(a.dx[d] + o.X + cc), rx = S(0);
+      return;
+    }
+  }
   const long i = a.axis_tab ? (long)(o.A[d] + pd) : o.X + cc;
   if constexpr (sizeof(S) == 8) {
     const double2 v = __ldg((const double2*)a.xr[d] + i);
@@ -383,7 +390,7 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
     }
     T dxv[NDIM], rxv[NDIM];  // the cell widths and their reciprocals
 #pragma unroll
-    for (int d = 0; d < NDIM; ++d) width_at(a, o, d, pos[d], cg, dxv[d], rxv[d]);
+    for (int d = 0; d < NDIM; ++d) width_at<FAST>(a, o, d, pos[d], cg, dxv[d], rxv[d]);
     constexpr T r12 = T(1.0 / 12.0);
     // gradient4 (src/vacgrid.t:684): -(q(+2) - 8(q(+1)-q(-1)) - q(-2))/dx/12, zero on
     // the first and last two mesh cells along its dimension (:690-709)
@@ -538,7 +545,7 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
               } else {
                 if (in) {
                   T dxkj, rxkj;
-                  width_at(a, o, k, pos[k], jg, dxkj, rxkj);
+                  width_at<FAST>(a, o, k, pos[k], jg, dxkj, rxkj);
                   T njl, njr;
                   nus(PR::v(l, k), k, j, dxkj, njl, njr);
                   const T gC = z1[k] ? T(0) : qdiv<FAST>(ldt<TILE>(q, j + sk) - ldt<TILE>(q, j - sk), dxkj, rxkj) / T(2);
@@ -582,7 +589,7 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
               } else {
                 if (in) {
                   T dxkj, rxkj;
-                  width_at(a, o, k, pos[k], jg, dxkj, rxkj);
+                  width_at<FAST>(a, o, k, pos[k], jg, dxkj, rxkj);
                   T njl, njr;
                   nus(PR::b(l, k), k, j, dxkj, njl, njr);
                   const T gC = z1[k] ? T(0) : qdiv<FAST>(ldt<TILE>(q, j + sk) - ldt<TILE>(q, j - sk), dxkj, rxkj) / T(2);
@@ -658,7 +665,7 @@ __device__ __forceinline__ void update_cell(const Stage2Args& a, const Geom& g, 
             const int sj = st[j];
             T dxn, rxn;
             const int row = (j != d && ghost) ? 1 + 2 * (d < j ? d : d - 1) + (sg > 0 ? 1 : 0) : 0;
-            width_at(a, o, j, row * g.n[j] + pos[j] + (j == d ? sg : 0), (long)n, dxn, rxn);
+            width_at<FAST>(a, o, j, row * g.n[j] + pos[j] + (j == d ? sg : 0), (long)n, dxn, rxn);
             const T gr = qdiv<FAST>(-(Bat(k, n + sj) - Bat(k, n - sj)), dxn, rxn) / T(2);
             J[i] = (l == 1) ? J[i] + gr : J[i] - gr;
           }
@@ -913,7 +920,7 @@ __device__ __forceinline__ void cross_cell(const Stage2Args& a, const Geom& g, c
     const int sk = st[k];
     const bool z1 = (a.zero1[k][0] && pos[k] == g.lo[k]) || (a.zero1[k][1] && pos[k] == g.hi[k]);
     T dxk, rxk;
-    width_at(a, o, k, pos[k], (long)c, dxk, rxk);
+    width_at<FAST>(a, o, k, pos[k], (long)c, dxk, rxk);
 #pragma unroll
     for (int l = 0; l < NDIM; ++l) {
       if (l == k) continue;

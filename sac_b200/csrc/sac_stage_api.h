@@ -51,7 +51,8 @@ struct Stage2Args {
   const void* X;     // S[n_cross][N] cross-derivative half-sums (single grid), or nullptr
   // cell widths with their reciprocals, (dx, 1/dx) pairs of S per dimension: one row
   // of entries per index along it where the width varies along its own dimension alone
-  // (axis_tab, every Cartesian grid; the rows of width_row), else one per cell [N]
+  // (axis_tab, every Cartesian grid; the rows of width_row), else one per cell [N]; in
+  // FP64 nullptr where the memory did not reach (then general)
   const void* xr[3];
   int axis_tab;
   // brick flags of the FP64 single grid (k_face): a brick of 8 cells per dimension is
@@ -59,7 +60,7 @@ struct Stage2Args {
   // reach it then take the divides; brick strides fst
   unsigned char* flags;
   int fst[3];
-  const double* dx[3];  // cell widths per cell (the batch's getdt_courant)
+  const double* dx[3];  // cell widths per cell (grids without the table, the batch's getdt_courant)
   // every cell takes the update's general form: a split sweep (dmin..dmax), a partial
   // variable list (iwmask), or widths, eta or the step out of range
   int general;

@@ -47,3 +47,10 @@ def test_the_gemm_epilogue_gathers_its_warp_before_each_load():
     src = _code(os.path.join("fno", "fno_gemm.cuh"))
     turn = src[src.index("cc < BN"):]
     assert turn.index("__syncwarp()") < turn.index("tcgen05.ld") < turn.index("continue")
+
+
+@pytest.mark.parametrize("name", ["sac_gpu.cu", "sac_batch.cu"])
+def test_setting_a_grid_makes_no_pinned_allocation(name):
+    """A pinned allocation and its release take over a millisecond each, several times the
+    whole set-up of a small grid; what getdt brings to the host needs none."""
+    assert not re.search(r"cudaMallocHost|cudaHostAlloc", _code(name))

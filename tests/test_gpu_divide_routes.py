@@ -23,8 +23,8 @@ def _steps_equal(P, nsteps, dt_frac=0.1, **sweep):
     c.lib.sac_general_kernels.argtypes = [abi.ctypes.c_void_p]
     n, route = 2 * P.ndir + 2, []
     dt = dt_frac * o.getdt(0)
-    c.getdt(0)
     for it in range(nsteps):
+        c.getdt(it)  # brings the count that chooses the kernels
         for x in (c, o):
             x.advect(dt, it * dt, it, **sweep)
         got, want = c.download(), o.download()
