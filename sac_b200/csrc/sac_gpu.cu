@@ -65,14 +65,14 @@ struct sac_ctx {
   void* D = nullptr;
   void* F = nullptr;
   void* R = nullptr;
-  void* X = nullptr;  // cross-derivative half-sums (k_cross), allocated with hyperdiffusion
+  void* X = nullptr;  // cross-derivative half-sums (k_cross), with hyperdiffusion; FP32: stg
   double* dx = nullptr;
   void* xr = nullptr;  // cell widths with their reciprocals (Stage2Args::xr)
   long xr_off[3] = {0, 0, 0};  // pairs before dimension d's
   int axis_tab = 0;
   bool widths_ok = true;  // the widths are in qdiv's range, with their reciprocals in xr
   double* drv = nullptr;
-  double* stg = nullptr;  // FP64 staging block for FP32 upload/download
+  double* stg = nullptr;  // FP64 staging block for FP32 upload/download; between them X
   double drvA = 0.0;
   // 0 maxnu, 1 courant, 2 the warps counted by a probing stage (32 bits), 3..5 ctot; then
   // the FP64 stage's brick flags (one memset clears ctot and the flags)
@@ -217,6 +217,7 @@ bool grav_module(int u) {
 void release(sac_ctx* c) {
   for (auto& p : c->P)
     if (p) cudaFree(p), p = nullptr;
+  if (c->X == (void*)c->stg) c->X = nullptr;
   for (void* p : {(void*)c->BG, c->D, c->F, c->R, c->X, (void*)c->dx, c->xr, (void*)c->drv,
                   (void*)c->stg, (void*)c->red, (void*)c->kp, (void*)c->fixB, (void*)c->d_type,
                   (void*)c->d_fixed})
@@ -981,8 +982,15 @@ sac_status sac_set_grid(sac_ctx* c, int ndim, int ndir, const int ixGhi[3], cons
   CK(cudaMalloc(&c->D, c->es * (ndir + 3) * N));
   CK(cudaMalloc(&c->F, c->es * (size_t)ndim * g.np * N));
   CK(cudaMalloc(&c->R, c->es * (size_t)nr_pairs(ndim) * N));
-  if (visc_on(c) && ndim > 1)  // the update reads them (k_cross)
+  // the cross terms that the update reads (k_cross): of a stage, so that FP32, which
+  // stages uploads and downloads in a block of its own, keeps them there (16 or 48 of
+  // its 48 to 64 bytes per cell)
+  if (c->prec == SAC_PREC_FP32) {
+    CK(cudaMalloc(&c->stg, std::max(sizeof(double) * g.np, c->es * n_cross(ndim)) * N));
+    if (visc_on(c) && ndim > 1) c->X = c->stg;
+  } else if (visc_on(c) && ndim > 1) {
     CK(cudaMalloc(&c->X, c->es * (size_t)n_cross(ndim) * N));
+  }
   CK(cudaMalloc(&c->dx, sizeof(double) * ndim * N));
   // the widths' table, where they vary along their own dimension alone
   c->axis_tab = widths_on_axes(g.n, g.lo, g.hi, ndim, N, hdx.data()) ? 1 : 0;
@@ -1004,7 +1012,6 @@ sac_status sac_set_grid(sac_ctx* c, int ndim, int ndir, const int ixGhi[3], cons
                        cudaMemcpyHostToDevice, c->stream));
   }
   if (!hdrv.empty()) CK(cudaMalloc(&c->drv, sizeof(double) * 2 * N));
-  if (c->prec == SAC_PREC_FP32) CK(cudaMalloc(&c->stg, sizeof(double) * g.np * N));
   c->nflags = 0;
   if (c->prec == SAC_PREC_FP64) {
     c->nflags = 1;
