@@ -380,9 +380,9 @@ __global__ void k_sumsq(const float* __restrict__ g, long n, float* out) {
 
 // loss = mean (y - t)^2 over the first cout channels; dy = 2 (y - t) / n as BF16
 // in a buffer of cpad >= cout channels (the padding channels are zeroed)
-// The loss is one atomic per warp: FP32 additions to a running total round by the size
-// of each addend, whatever their order, so another grouping (one per block, 67 -> 10 us
-// for 16 samples of 256 x 256) moved it by up to 2e-5, as much as FP32 results may differ
+// The loss is one atomic per warp.  One per block takes 10 us instead of 67 for 16 samples
+// of 256 x 256, but an FP32 sum of so many addends rounds with their grouping, and the loss
+// moved by up to 2e-5 of itself
 __global__ void k_mse(const float* __restrict__ y, const bf16* __restrict__ t, bf16* __restrict__ dy, float* loss,
                       int B, int cout, int cpad, long P, float inv_n) {
   float s = 0.f;
@@ -702,7 +702,8 @@ int forward(sac_fno* n, const bf16* x, float* y, int B, bool train) {
   n->Blast = B;
   // where the shape allows it the lift and the layers' pixel stages run row by row,
   // with the next layer's DFT along f in the same kernel (fno_row.cuh)
-  const bool rows = row_ok(n) && ((uintptr_t)x & 15) == 0;
+  const bool rows = row_ok(n);
+  if (!aligned16p(x)) return fail(n, "sac_fno_gemm: operands must be 16-byte aligned");  // the lift of either kind
   if (rows) {
     RowArgs a = row_args(n, B);
     a.in = x;
@@ -959,7 +960,6 @@ int bias_grad(sac_fno* n, const bf16* d, int C, float* out, int B) {
   return 0;
 }
 
-// dy: [B][cpad][P] bf16 (gradient of the loss w.r.t. y; padding channels zero)
 // one k_wgrad launch: persistent, one CTA per SM
 template <int R, int C, bool TR>
 int wgrad_launch(sac_fno* n, const bf16* d, const bf16* in, float* gw, float* gb, int B) {
@@ -992,6 +992,7 @@ int layer_grad(sac_fno* n, const bf16* d, int R, const bf16* in, int C, float* g
   return rc ? rc : bias_grad(n, d, R, gb, B);
 }
 
+// dy: [B][cpad][P] bf16 (gradient of the loss w.r.t. y; padding channels zero)
 int backward(sac_fno* n, const bf16* dy) {
   const int B = n->Blast, S = n->S, F = n->F, W = n->W, H = n->H, cpad = n->cpad;
   const long P = n->P;
@@ -1346,8 +1347,10 @@ int sac_fno_create(const sac_fno_config* cfg, sac_fno** out) {
   FK(cudaMalloc(&n->dzt, sizeof(bf16) * B * W * kJ * kR));
   FK(cudaMalloc(&n->dpt, sizeof(float) * B * W * kJ * kR));
   FK(cudaMalloc(&n->yb, sizeof(bf16) * B * W * n->S * kJ));
-  FK(cudaMalloc(&n->spec, sizeof(float) * BWP));
-  if (!row_ok(n)) FK(cudaMalloc(&n->dvacc, sizeof(float) * BWP));
+  if (!row_ok(n)) {  // the row kernel keeps both sums in TMEM
+    FK(cudaMalloc(&n->spec, sizeof(float) * BWP));
+    FK(cudaMalloc(&n->dvacc, sizeof(float) * BWP));
+  }
   FK(cudaMalloc(&n->dz, sizeof(bf16) * BWP));
   FK(cudaMalloc(&n->dz2, sizeof(bf16) * BWP));
   FK(cudaMalloc(&n->scal, sizeof(float) * 4));

@@ -145,3 +145,19 @@ def test_no_samples_and_no_state_channels_are_no_work():
     torch.cuda.synchronize()
     assert bool((st == 1).all()) and bool((x == 1).all())
     net.close()
+
+
+def test_an_unaligned_input_is_refused():
+    """As by the GEMM of the lift: status 1, whichever kernels serve the network."""
+    from sac_b200 import fno_abi
+
+    for F in (72, 264):
+        net = _net(56, F, 1)
+        x = torch.zeros(16 * 56 * F + 1, dtype=torch.bfloat16, device="cuda")[1:]
+        y = torch.zeros(6, 56, F, device="cuda")
+        torch.cuda.synchronize()
+        for run in (net.forward, net.infer):
+            with pytest.raises(fno_abi.FnoError) as e:
+                run(x.data_ptr(), y.data_ptr(), 1)
+            assert "status 1" in str(e.value)
+        net.close()

@@ -40,3 +40,21 @@ def test_fp32_grid_holds_its_fields_and_no_more(nx, ndir, sheared):
     c.close()
     # fixB and the small tables, and the allocations' rounding to 2 MB
     assert used <= per_cell * cells * 1.02 + 40e6, (used, per_cell * cells)
+
+
+def test_a_network_of_the_row_kernel_holds_no_fp32_intermediates():
+    """Activations, pre-activations, dz and its twin (BF16), the three hidden buffers (BF16),
+    the transforms and the parameters: no FP32 buffer of width x pixels."""
+    from sac_b200 import fno_abi
+
+    B, S, F, W, L, H, kJ, kR = 8, 256, 256, 32, 4, 128, 48, 96
+    bwp = B * W * S * F
+    fno_abi.Net(S=S, F=F, max_batch=1, seed=1).close()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    net = fno_abi.Net(S=S, F=F, max_batch=B, seed=1)
+    used = free - torch.cuda.mem_get_info()[0]
+    npar = net.nparam
+    net.close()
+    want = 2 * bwp * ((L + 1) + L + 2 + 3 * H // W) + 4 * 2 * B * W * kJ * S + (4 * (L + 1) + 2 * 2) * B * W * kJ * kR
+    assert used <= (want + 18 * npar) * 1.02 + 40e6, (used, want + 18 * npar)
