@@ -199,7 +199,7 @@ void sac_destroy(sac_ctx* c);
 /* ---- library extensions: no counterpart in the reference ------------------
  * Stream selection lets a host run the path on its own CUDA stream; profiling
  * brackets every kernel launch with CUDA events on that stream. */
-#define SAC_K_STAGE 0   /* k_update: the per-cell stage update */
+#define SAC_K_STAGE 0   /* k_update: the per-cell stage update; k_step1d: a whole step of a 1D grid */
 #define SAC_K_PREP 1    /* k_face: derived fields, fluxes, c_tot */
 #define SAC_K_BOUND 2   /* k_bound: ghost-cell resolve */
 #define SAC_K_COURANT 3 /* getdt_courant reduction */

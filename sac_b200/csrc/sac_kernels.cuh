@@ -92,29 +92,22 @@ __device__ __forceinline__ float div_rn(float a, float b) { return __fdiv_rn(a, 
 // n times the sign of d, which n * d gives.  The shortcut is taken only where d
 // is finite and nonzero.  An FP64 division whose numerator is zero leaves the
 // fast path of the divide (measured on B200: 3.6x the time of one with a normal
-// numerator); k_face divides the momenta, which are exactly zero over most of a
-// run that starts from rest, by rho'+rhob.  FP32 storage keeps its plain
-// (approximate) division.
-template <typename T>
-__device__ __forceinline__ T dvs(T n, T d) {
-  if constexpr (sizeof(T) == 8) {
-    if (n == T(0) && d != T(0) && fabs(d) <= 1.7976931348623157e308) return n * d;
-  }
-  return n / d;
-}
+// numerator); k_face's general form divides the momenta, which are exactly zero over
+// much of a run that starts from rest, by rho'+rhob.
 __device__ __forceinline__ double dvs_rn(double n, double d) {
   if (n == 0.0 && d != 0.0 && fabs(d) <= 1.7976931348623157e308) return __dmul_rn(n, d);
   return __ddiv_rn(n, d);
 }
-__device__ __forceinline__ float dvs_rn(float n, float d) { return __fdiv_rn(n, d); }
 
 // ---- divisions by a divisor whose reciprocal is at hand -------------------
 // Correctly rounded n / d from r = RN(1/d): q = RN(n r), e = n - q d, RN(q + e r)
 // (Markstein, "Computation of elementary functions on the IBM RISC System/6000
 // processor", 1990): one multiply and two FMAs instead of the divide's reciprocal
 // iteration, and no slow path, whose branch keeps the loads behind it from being
-// issued ahead.  e has to be exact and q normal: n zero (the quotient is then a zero,
-// whose sign may differ from the divide's) or at least 2^-969 in magnitude.
+// issued ahead.  e has to be exact and the quotient normal: n zero (the quotient is then
+// a zero, whose sign may differ from the divide's), or at least 2^-969 in magnitude with
+// n / d at least 2^-1022 (for d = 12, whose last bits are zeros, the latter is enough).
+// Below that the last bit may differ.
 __device__ __forceinline__ double div_markstein(double n, double d, double r) {
   const double q = __dmul_rn(n, r);
   const double e = __fma_rn(-q, d, n);
@@ -140,13 +133,21 @@ __device__ __forceinline__ float qdiv(float n, float d, float r) {
 }
 
 // A field value outside {0} and [2^-200, 2^100) in magnitude, NaN and Inf included.
-// With a cell's and its stencil's fields inside, the total density nonzero and c_tot
-// and the widths in their ranges, every numerator of the stage is zero or at least
-// 2^-859: the smallest are gradient4's of the energy flux (products of three fields,
-// 2^-600, over a density of 2^100, with 53 bits of cancellation in the product sum, in
-// the flux and in the difference) and the differences of a momentum times a viscous
-// flux (2^-200 * 2^-593: a velocity difference 2^-353 over a width of 2^40, c_tot
-// 2^-100, setnu's quotient 2^-60 and a width 2^-40).
+// With a cell's and its stencil's fields inside, the total density in [2^-100, 2^100) and
+// c_tot and the widths in their ranges, the numerators of the stage are zero or at least
+// (a sum cancels to the last bit of its smallest term at the least, 2^-53 of it)
+//   over the density: 2^-807 (energy flux: m_d p', p' from m^2/rho, 2^-754, in its sum);
+//   over a width: 2^-960 (a difference of such fluxes, 2^-907 over the largest density),
+//     2^-904 (momentum times viscous flux: a mean of momenta 2^-253; a velocity difference
+//     2^-353 over 2^40, c_tot 2^-105, a quotient of setnu of 2^-60, a width of 2^-40);
+//   over 12: 2^-1000 (the flux difference over a width).
+// Two kinds can be smaller.  getcmax's 4 cs2 B_d^2, B_d and cs2 both by cancellation: its
+// error then is the last bit of a term below 2^-822 under a square root beside cf2^2,
+// which counts only where every wave speed of the mesh is below 2^-205, and there c_tot is
+// out of its range (9e7 random cells of that kind: no quotient differed).  And viscous
+// fluxes whose quotient of setnu is below 2^-60, third differences that cancel to less
+// than the first ones' last bits: the last bit of a quotient below 2^-929, which shows
+// only in a variable whose cell holds nothing larger.
 constexpr unsigned kRangeLo = (1023u - 200u) << 20, kRangeHi = (1023u + 100u) << 20;
 __device__ __forceinline__ bool out_of_range(double x) {
   const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu;

@@ -9,7 +9,7 @@
 //            arithmetic (face_eval);
 //   phase 2  setnu's face quotients along x and along y at the faces the update
 //            and its inline cross terms read (c and c - s_k, at the tile's cells
-//            and one cell around) -- the k_nu arithmetic (face_quotient), with
+//            and one cell around) -- the k_nu arithmetic (face_maxima, face_ratio), with
 //            c_tot of the stage from kb_ctot;
 //   phase 3  the update of each cell (update_cell in its tile form: the stencil
 //            fields from shared memory, the cell's own base, background, widths,
