@@ -476,14 +476,16 @@ sac_status advect1_t(sac_ctx* c, const std::string& method, double qdt, int dmin
 }
 
 // Whether a 'fourstep' step runs as one launch (k_step1d): a 1D grid of 64 cells (below,
-// a CTA's segment would not hold setnu's mirrored cells) to what fits in the cluster's
-// shared memory (about 17000 in FP64), the default sources, an unsplit sweep over all
-// variables
+// a CTA's segment would not hold setnu's mirrored cells) to where the launches, which have
+// the whole chip, overtake eight SMs; the default sources, an unsplit sweep over all
+// variables.  getdt + step, one launch against the launches, us: 71 / 121 at 804 cells,
+// 102 / 122 at 8004, 128 / 123 at 12004 (ndir 2), 129 / 130 at 10004 (ndir 3); FP32
+// 119 / 120 at 17004
 bool step1d_ok(const sac_ctx* c, const std::string& m, unsigned mask) {
   const Geom& g = c->g;
   return g.ndim == 1 && m == "cd4" && mask == (1u << g.np) - 1u && !c->regions && !c->par.smallfix &&
-         !(c->par.sourceunsplit && std::fabs(c->par.eta) > smalldouble) && g.n[0] >= 64 && g.n[0] < 30000 &&
-         step1d_smem(g.np, g.n[0], c->es) <= kStep1dSmem;
+         !(c->par.sourceunsplit && std::fabs(c->par.eta) > smalldouble) && g.n[0] >= 64 &&
+         g.n[0] <= step1d_most(c->es);
 }
 
 template <typename S>

@@ -137,18 +137,22 @@ inline long count_warps(const Geom& g) {
 }
 
 // a whole RK4 step of a small 1D grid in one launch (sac_step1d.cuh): the four stages'
-// arguments and boundary fills; the largest shared memory such a grid may take
+// arguments and boundary fills
 struct Step1dArgs {
   Stage2Args st[4];
   BcArgs bc[4];
 };
-constexpr int kStep1dCtas = 8, kStep1dSmem = 220 * 1024;
-// the cells of one CTA; its shared memory: the stencil fields of np advanced variables
-// and a byte for each cell of the segment and three to either side
-__host__ __device__ inline int step1d_segment(int n) { return (n + kStep1dCtas - 1) / kStep1dCtas; }
-inline int step1d_smem(int np, int n, size_t es) {
+constexpr int kStep1dCtas = 8;
+// the largest such grid by storage size (step1d_ok), the cells of one CTA, and its shared
+// memory: the stencil fields of np advanced variables and a byte for each cell of the
+// segment and three to either side; the kernel's limit on it
+constexpr int step1d_most(size_t es) { return es == 8 ? 10000 : 17000; }
+__host__ __device__ constexpr int step1d_segment(int n) { return (n + kStep1dCtas - 1) / kStep1dCtas; }
+constexpr int step1d_smem(int np, int n, size_t es) {
   return (5 + (np - 1) + 3) * (step1d_segment(n) + 6) * (int)es + step1d_segment(n) + 6;
 }
+constexpr int kStep1dSmem = step1d_smem(8, step1d_most(8), 8);
+static_assert(step1d_smem(8, step1d_most(4), 4) <= kStep1dSmem && kStep1dSmem <= 220 * 1024, "one limit for both");
 template <typename S>
 cudaError_t launch_step1d(const Step1dArgs& p, cudaStream_t st);
 extern template cudaError_t launch_step1d<double>(const Step1dArgs&, cudaStream_t);

@@ -70,3 +70,24 @@ def test_fp32_steps_stay_in_the_twin_envelope(nx):
     Q.params.precision = params.PREC_FP32
     w, _, _ = _steps(Q, abi.Context, 4)
     assert np.isfinite(w).all()
+
+
+@pytest.mark.parametrize("fp32,most", [(False, 10000), (True, 17000)])
+def test_the_largest_grid_of_one_launch_and_the_next(fp32, most):
+    """The last grid (ghosts included) that takes the one launch and the first that takes
+    the launches: FP64 equals the oracle, FP32 the other route's envelope."""
+    from oracle.oracle import Oracle
+
+    abi.load()[0].sac_kernel_launches.argtypes = [abi.ctypes.c_void_p]
+    abi.load()[0].sac_kernel_launches.restype = abi.ctypes.c_long
+    for n in (most, most + 1):
+        P = problems.random_problem((n - 4,), ndir=3, seed=64, types=["periodic", "periodic"])
+        if fp32:
+            err, twin = _util.fp32_twin(P, 2)
+            assert (err <= 1e-5).all() or (err <= 150 * twin).all(), (err, twin)
+            P.params.precision = params.PREC_FP32
+        got, dts, k = _steps(P, abi.Context, 1)
+        assert (k < 10) == (n == most), (n, k)
+        if not fp32:
+            want, _, _ = _steps(P, Oracle, 1, dts)
+            np.testing.assert_array_equal(got, want)
