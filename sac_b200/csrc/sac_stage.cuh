@@ -81,7 +81,7 @@ __device__ __forceinline__ void width_at(const Stage2Args& a, const Offs& o, int
 // of the same (launch_update).
 template <int NDIM, int NDIR, typename S, class DOut, class FOut>
 __device__ __forceinline__ bool face_eval(const Stage2Args& a, const Offs& o, long c, bool mesh, double gamma,
-                                          double* cm, unsigned fdims, bool test, DOut&& dout, FOut&& fout) {
+                                          double* cm, unsigned fdims, bool test, DOut&& dout, FOut&& fout, bool divides = false) {
   constexpr int E = NDIR + 1;
   auto W = [&](int iw) { return (const S*)a.fW[iw] + o.P; };
   auto BG = [&](int i) { return a.fBG[i] + o.B; };
@@ -201,7 +201,9 @@ __device__ __forceinline__ bool face_eval(const Stage2Args& a, const Offs& o, lo
       }
     }
   };
-  if (bad || (sizeof(S) == 8 && a.quiet))
+  // one form per warp (the lanes that are here): a mixed one would run both
+  const bool divide = bad || (sizeof(S) == 8 && (divides || a.quiet));
+  if (sizeof(S) == 8 ? __any_sync(__activemask(), divide) != 0 : divide)
     body(std::false_type{});
   else
     body(std::true_type{});

@@ -109,8 +109,10 @@ __device__ __forceinline__ void stage2d_tile(const BatchStageArgs& b, int t, uns
       const unsigned fd = ((by >= L::FX_R0 && by < L::FX_R0 + L::FX_NR && bx >= H - 2 && bx < H + TX + 2) ? 1u : 0u) |
                           ((bx >= H && bx < H + TX && by >= L::FY_R0 && by < L::FY_R0 + L::FY_NR) ? 2u : 0u);
       double cm[NDIM];
+      // once a cell of this warp's is out of range the tile divides: so does the warp, untested
+      const bool divides = sizeof(S) == 8 && __any_sync(__activemask(), bad);
       bad |= face_eval<NDIM, NDIR, S>(
-          b.a, I.o, c, false, b.a.gamma, cm, fd, true,
+          b.a, I.o, c, false, b.a.gamma, cm, fd, !divides,
           [&](int i, S v) {
             if (i == 0) sm[L::P_OFF + L::P_RT * BW * BH + idx] = v;
             else if (i <= NDIM) sm[L::P_OFF + (L::P_V + i - 1) * BW * BH + idx] = v;
@@ -121,7 +123,8 @@ __device__ __forceinline__ void stage2d_tile(const BatchStageArgs& b, int t, uns
               sm[L::FX_OFF + L::fslot(0, iw) * BW * L::FX_NR + (by - L::FX_R0) * BW + bx] = v;
             else
               sm[L::FY_OFF + L::fslot(1, iw) * BW * L::FY_NR + (by - L::FY_R0) * BW + bx] = v;
-          });
+          },
+          divides);
       const S* w0 = (const S*)b.a.fW[0] + I.o.P;
       sm[L::P_OFF + L::P_RHO * BW * BH + idx] = w0[c];
 #pragma unroll
@@ -223,8 +226,10 @@ __device__ __forceinline__ void stage2d_tile(const BatchStageArgs& b, int t, uns
 }
 
 // resident CTAs per SM the fused stage is compiled for: FP64 2 (its 97.6 KB of
-// tile memory allows no more; 128 registers), FP32 4 (64 registers, no spills for
-// ndir 2)
+// tile memory allows no more; 128 registers), at 16 x 8 as many as its tile memory
+// allows (56 KB for ndir 2, 64 for 3: 128 and 168 registers without spills; left to the
+// compiler it took 174 and 184, and 24 vortices 412 us per step instead of 386, 24
+// tubes from rest 1118 instead of 916), FP32 4 (64 registers, no spills for ndir 2)
 #ifndef SAC_STAGE2D_MINB_F64
 #define SAC_STAGE2D_MINB_F64 2
 #endif
@@ -232,7 +237,9 @@ __device__ __forceinline__ void stage2d_tile(const BatchStageArgs& b, int t, uns
 #define SAC_STAGE2D_MINB_F32 4
 #endif
 template <int NDIR, typename S, int TX, int TY>
-__global__ void __launch_bounds__(TX * TY, sizeof(S) == 4 ? SAC_STAGE2D_MINB_F32 : SAC_STAGE2D_MINB_F64)
+__global__ void __launch_bounds__(TX * TY, sizeof(S) == 4   ? SAC_STAGE2D_MINB_F32
+                                           : TX * TY < 256 ? (NDIR == 2 ? 4 : 3)
+                                                           : SAC_STAGE2D_MINB_F64)
     kb_stage2d(const __grid_constant__ BatchStageArgs b) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ double shred[32];
