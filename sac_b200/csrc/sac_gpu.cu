@@ -1355,10 +1355,10 @@ static sac_status getdt_impl(sac_ctx* c, double* dt, int it, bool static_scratch
       else
         launch(0.0);
       }
-      // both maxima and the count in one copy and one wait; courant starts the next call at zero
+      // both maxima and the count in one copy, which to pageable memory returns when it is
+      // done (no wait for what follows it); courant starts the next call at zero
       CK(cudaMemcpyAsync(c->h_red, c->red, sizeof(c->h_red), cudaMemcpyDeviceToHost, c->stream));
       CK(cudaMemsetAsync(c->red + 1, 0, sizeof(unsigned long long), c->stream));
-      CK(cudaStreamSynchronize(c->stream));
       have_maxnu = true;
       c->count_taken = false;
       double courantmax;
