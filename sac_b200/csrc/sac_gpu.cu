@@ -45,9 +45,10 @@ constexpr double bigdouble = 1.0e99, smalldouble = 1.0e-99;
 constexpr long quiet_percent(int ndim, bool sources) {
   return ndim == 3 ? (sources ? 50 : 23) : (ndim == 2 && sources ? 25 : 100);
 }
-// ... as counted in one stage of this many, whose k_face tests every field in the general
-// form's steps too (a launch of 4 to 13 us)
-constexpr unsigned kProbeStages = 16;
+// ... as counted in some stages (k_count_divides: 4 to 13 us, and k_face tests every field
+// in the general form's steps too): at first and after a change the stages 0, 1, 3, 7, 15
+// from there, then one of this many
+constexpr long kProbeStages = 16;
 }
 
 struct sac_ctx {
@@ -83,7 +84,8 @@ struct sac_ctx {
   unsigned long long h_red[3] = {0, 0, 0};
   bool count_taken = false;
   size_t nflags = 0;  // bytes of flags (0: FP32)
-  unsigned stages = 0;  // stages since sac_set_grid that could have probed
+  long stages = 0, probe_at = 0, probe_gap = 1;  // stages so far, the next that counts
+  int was_quiet = 0;
   unsigned long long* kp = nullptr;   // keeppositive's words (smallfix only), see k_keeppos_scan
   int it_now = 0;                     // the step number last passed to sac_getdt or sac_advect
   double* fixB = nullptr;
@@ -397,7 +399,13 @@ Stage2Args stage_args(sac_ctx* c, bool flux, double qdt, int dmin, int dmax, dou
   const long quiet = quiet_percent(g.ndim, a.res_on || a.divb_on);
   if (quiet < 100 && c->nflags && !a.general) {
     a.quiet = 100L * (long)(unsigned)c->h_red[2] > quiet * count_warps(g) ? 1 : 0;
-    a.probe = c->stages++ % kProbeStages == 0 ? 1 : 0;
+    if (a.quiet != c->was_quiet) c->probe_gap = 1, c->was_quiet = a.quiet;
+    a.probe = c->stages >= c->probe_at ? 1 : 0;
+    if (a.probe) {
+      c->probe_at = c->stages + c->probe_gap;
+      c->probe_gap = std::min(2 * c->probe_gap, kProbeStages);
+    }
+    ++c->stages;
   }
   a.driver = DRV_NONE;
   if (c->par.sourceunsplit && c->drv) {
@@ -1021,7 +1029,7 @@ sac_status sac_set_grid(sac_ctx* c, int ndim, int ndir, const int ixGhi[3], cons
   }
   CK(cudaMalloc(&c->red, 6 * sizeof(unsigned long long) + c->nflags));
   CK(cudaMemsetAsync(c->red, 0, 6 * sizeof(unsigned long long) + c->nflags, c->stream));
-  c->stages = 0;
+  c->stages = c->probe_at = 0, c->probe_gap = 1, c->was_quiet = 0;
   std::memset(c->h_red, 0, sizeof(c->h_red));
   c->count_taken = false;
   if (c->par.smallfix) {
@@ -1231,6 +1239,7 @@ sac_status sac_upload(sac_ctx* c, const double* w) {
   CK(cudaMemcpyAsync(c->BG, w + (long)g.np * N, sizeof(double) * (g.nw - g.np) * N, cudaMemcpyHostToDevice,
                      c->stream));
   CK(cudaStreamSynchronize(c->stream));
+  c->probe_at = c->stages, c->probe_gap = 1;  // another state: count anew
   c->state_set = true;
   return SAC_OK;
 }

@@ -127,3 +127,12 @@ def test_fused_batch_stage_with_cells_out_of_range(shape):
         a.advance(1)
         f.advance(1)
         np.testing.assert_array_equal(f.download(), a.download())
+
+
+def test_a_state_that_leaves_rest_changes_kernels_in_a_step():
+    """At rest every field is zero or background, which is in range, and the driver is zero
+    in the step at t = 0; its far tail in the next is not. That step counts it and those
+    behind it divide everywhere."""
+    P = problems.stratified((48, 40, 40))
+    P.params.userpar[4], P.params.userpar[6] = 0.03, 0.03  # out of range from 0.35 on
+    assert _steps_equal(P, 4, dt_frac=0.5) == [0, 0, 1, 1]
