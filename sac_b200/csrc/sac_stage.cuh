@@ -871,18 +871,15 @@ template <int NDIM>
 __device__ __forceinline__ bool row_out_of_range(const Stage2Args& a, const int pos[3]) {
   const Geom& g = a.g;
   const int lane = threadIdx.x & 31, x0 = pos[0] - lane;
-  const int i = lane % 6, j = lane / 6 % 2, k = lane / 12;  // 35 + 3 cells touch 6 bricks, 7 cells 2
-  const int b0 = max((x0 - 3) >> 3, 0) + i;
+  const int j = lane >> 3 & 1, k = lane >> 4;  // 32 + 6 cells touch up to 6 bricks, 7 cells 2
+  const int b0 = max((x0 - 3) >> 3, 0) + (lane & 7);
   bool bad = false;
   if (b0 <= min(x0 + 34, g.n[0] - 1) >> 3 && j < (NDIM > 1 ? 2 : 1) && k < (NDIM > 2 ? 2 : 1)) {
     const int b1 = NDIM > 1 ? min(max(pos[1] + (j ? 3 : -3), 0), g.n[1] - 1) >> 3 : 0;
     const int b2 = NDIM > 2 ? min(max(pos[2] + (k ? 3 : -3), 0), g.n[2] - 1) >> 3 : 0;
     bad = __ldg(a.flags + b0 + a.fst[1] * b1 + a.fst[2] * b2) != 0;
   }
-  if (a.visc_on) {
-#pragma unroll
-    for (int d = 0; d < NDIM; ++d) bad = bad || ctot_out_of_range(a.ctot[d]);
-  }
+  if (a.visc_on && lane < NDIM) bad = bad || ctot_out_of_range(a.ctot[lane]);
   return __any_sync(0xffffffffu, bad);
 }
 
