@@ -24,7 +24,7 @@
 // Measured (B200, 64 samples of 256 x 256; a middle layer moves 268 MB in, 268 MB out
 // and 50 MB of T): 225 us, against 454 + 139 for its GEMMs before; the lift 156 us, the
 // last layer 159 (333 each).  It is bound by the epilogue's issue slots and the
-// latency of its turn (43 % of the slots used); 8 warps per SM took 293 us, and 487
+// latency of its turn (43 % of the slots used, 38 % at 16 samples); 8 warps per SM took 293 us, and 487
 // with 64-bit divisions in the row's indices, which are now stepped.
 // Every mbarrier wait is bounded; on time-out the CTA sets bit 0 of the error word,
 // drains its copies and MMAs, frees its TMEM and returns.

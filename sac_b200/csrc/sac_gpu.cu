@@ -45,7 +45,7 @@ constexpr double bigdouble = 1.0e99, smalldouble = 1.0e-99;
 constexpr long quiet_percent(int ndim, bool sources) {
   return ndim == 3 ? (sources ? 50 : 23) : (ndim == 2 && sources ? 25 : 100);
 }
-// ... as counted in some stages (k_count_divides: 4 to 13 us, and k_face tests every field
+// ... as counted in some stages (k_count_divides: 13 us at 128^3, and k_face tests every field
 // in the general form's steps too): at first and after a change the stages 0, 1, 3, 7, 15
 // from there, then one of this many
 constexpr long kProbeStages = 16;
