@@ -173,6 +173,11 @@ inline cudaError_t width_pairs_per_cell(const double* dx, long n, void** out, cu
   cudaError_t e = cudaMemGetInfo(&avail, &total);
   if (e != cudaSuccess || (sizeof(S) == 8 && avail < 2 * bytes)) return e;
   e = cudaMalloc(out, bytes);
+  if (sizeof(S) == 8 && e == cudaErrorMemoryAllocation) {
+    *out = nullptr;
+    cudaGetLastError();
+    return cudaSuccess;
+  }
   if (e != cudaSuccess) return e;
   k_width_pairs<S><<<592, 256, 0, st>>>(dx, (S*)*out, n);
   return cudaGetLastError();

@@ -136,3 +136,22 @@ def test_a_state_that_leaves_rest_changes_kernels_in_a_step():
     P = problems.stratified((48, 40, 40))
     P.params.userpar[4], P.params.userpar[6] = 0.03, 0.03  # out of range from 0.35 on
     assert _steps_equal(P, 4, dt_frac=0.5) == [0, 0, 1, 1]
+
+
+@pytest.mark.parametrize("sources", [False, True])
+@pytest.mark.parametrize("sheared", [False, True])
+@pytest.mark.parametrize("nx,ndir", [((60,), 2), ((43, 38), 2), ((19, 18, 17), 3)])
+def test_widths_out_of_range(nx, ndir, sheared, sources):
+    """Widths beyond the reciprocals' range divide everywhere, with the table per axis and,
+    where the axes are sheared, without any table."""
+    P = _problem(nx, ndir, sources)
+    P.params.grav[:] = [0.0, 0.0, 0.0]
+    x = P.x * 1e15
+    if sheared and len(nx) > 1:
+        x[..., 0] *= 1.0 + 0.03 * P.x[..., 1]
+    P.x = np.asfortranarray(x)
+    if sources:
+        P.params.eta *= 1e15
+    route = _steps_equal(P, 2)
+    if len(nx) > 1:
+        assert route == [1, 1]
