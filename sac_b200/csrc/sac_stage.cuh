@@ -201,9 +201,7 @@ __device__ __forceinline__ bool face_eval(const Stage2Args& a, const Offs& o, lo
       }
     }
   };
-  // one form per warp (the lanes that are here): a mixed one would run both
-  const bool divide = bad || (sizeof(S) == 8 && (divides || a.quiet));
-  if (sizeof(S) == 8 ? __any_sync(__activemask(), divide) != 0 : divide)
+  if (bad || (sizeof(S) == 8 && (divides || a.quiet)))
     body(std::false_type{});
   else
     body(std::true_type{});

@@ -109,8 +109,8 @@ __device__ __forceinline__ void stage2d_tile(const BatchStageArgs& b, int t, uns
       const unsigned fd = ((by >= L::FX_R0 && by < L::FX_R0 + L::FX_NR && bx >= H - 2 && bx < H + TX + 2) ? 1u : 0u) |
                           ((bx >= H && bx < H + TX && by >= L::FY_R0 && by < L::FY_R0 + L::FY_NR) ? 2u : 0u);
       double cm[NDIM];
-      // once a cell of this warp's is out of range the tile divides: so does the warp, untested
-      const bool divides = sizeof(S) == 8 && __any_sync(__activemask(), bad);
+      // once a cell of this thread's is out of range the tile divides: so do its other cells, untested
+      const bool divides = sizeof(S) == 8 && bad;
       bad |= face_eval<NDIM, NDIR, S>(
           b.a, I.o, c, false, b.a.gamma, cm, fd, !divides,
           [&](int i, S v) {
@@ -228,8 +228,8 @@ __device__ __forceinline__ void stage2d_tile(const BatchStageArgs& b, int t, uns
 // resident CTAs per SM the fused stage is compiled for: FP64 2 (its 97.6 KB of
 // tile memory allows no more; 128 registers), at 16 x 8 as many as its tile memory
 // allows (56 KB for ndir 2, 64 for 3: 128 and 168 registers without spills; left to the
-// compiler it took 174 and 184, and 24 vortices 412 us per step instead of 386, 24
-// tubes from rest 1118 instead of 916), FP32 4 (64 registers, no spills for ndir 2)
+// compiler it took 174 and 184, and 24 vortices 412 us per step instead of 382, 24
+// tubes from rest 1118 instead of 910), FP32 4 (64 registers, no spills for ndir 2)
 #ifndef SAC_STAGE2D_MINB_F64
 #define SAC_STAGE2D_MINB_F64 2
 #endif
